@@ -128,7 +128,7 @@ int uploadScene(const HostScene& h, SceneDev& s) {
       {h.tlas4.data(), bytesOf(h.tlas4), 0},     {h.blas4.data(), bytesOf(h.blas4), 0},
       {h.tlas4q.data(), bytesOf(h.tlas4q), 0},   {h.blas4q.data(), bytesOf(h.blas4q), 0},
       {h.mattex.data(), bytesOf(h.mattex), 0},   {h.tex.data(), bytesOf(h.tex), 0},
-      {h.vuv.data(), bytesOf(h.vuv), 0}};
+      {h.vuv.data(), bytesOf(h.vuv), 0},};
   size_t total = 0;
   for (auto& p : parts) {
     p.off = total;
@@ -142,6 +142,12 @@ int uploadScene(const HostScene& h, SceneDev& s) {
   char* base = static_cast<char*>(s.arena.base);
   for (auto& p : parts)
     if (p.bytes) CG_CUDA(cudaMemcpy(base + p.off, p.src, p.bytes, cudaMemcpyHostToDevice));
+  launchPermuteNodes(reinterpret_cast<Bvh4Node*>(base + parts[12].off), h.tlas4.size(), nullptr);
+  launchPermuteNodes(reinterpret_cast<Bvh4Node*>(base + parts[13].off), h.blas4.size(), nullptr);
+  launchPermuteNodes(reinterpret_cast<Bvh4QNode*>(base + parts[14].off), h.tlas4q.size(), nullptr);
+  launchPermuteNodes(reinterpret_cast<Bvh4QNode*>(base + parts[15].off), h.blas4q.size(), nullptr);
+  CG_CUDA(cudaGetLastError());
+  CG_CUDA(cudaStreamSynchronize(nullptr));
   SceneView& v = s.view;
   v.tlas = reinterpret_cast<const BvhNode*>(base + parts[0].off);
   v.blas = reinterpret_cast<const BvhNode*>(base + parts[1].off);

@@ -143,7 +143,7 @@ __device__ __forceinline__ int shadeKeyOf(const SceneView& sc, int32_t inst, boo
   if (inst < 0) return 0;
   if (cut) return 1;
   const uint4 meta = __ldg(reinterpret_cast<const uint4*>(sc.inst + inst) + 3);
-  return 2 + static_cast<int>((sc.mat[meta.y].volume >> kKindShift) & 15u);
+  return 2 + static_cast<int>(meta.z);  // DevInstance::kind
 }
 
 // The block's key counts of a keyed closest-hit launch (one shared array per
@@ -160,13 +160,13 @@ __device__ __forceinline__ void beginShadeKeys() {
 }
 
 // keys: 0 none, 1 keys for a level shaded before the depth cut, 2 after it.
-// Called by the lanes that finished a ray (one shared-memory atomic per
-// distinct key among them).
+// Called together by the lanes `lanes`, which finished a ray (one shared-memory
+// atomic per distinct key among them).
 __device__ __forceinline__ void writeShadeKey(const SceneView& sc, const WaveBuffers& wb, uint32_t i,
-                                              int32_t inst, int keys) {
+                                              int32_t inst, int keys, unsigned lanes) {
   const int key = shadeKeyOf(sc, inst, keys == 2);
   wb.shade_key[i] = static_cast<uint8_t>(key);
-  const unsigned peers = __match_any_sync(__activemask(), key);
+  const unsigned peers = __match_any_sync(lanes, key);
   if ((threadIdx.x & 31u) == static_cast<uint32_t>(__ffs(peers) - 1))
     atomicAdd(&blockKeyCounts()[key], static_cast<uint32_t>(__popc(peers)));
 }
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256, 4) k_extend(SceneView sc, WaveBuffers wb,
     HitRec h = trace<false, kCount, kNodes>(sc, o, d, MAXD, cnt, wb.status);
     wb.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.tri));
     wb.hit_inst[i] = h.inst;
-    if (keys) writeShadeKey(sc, wb, i, h.inst, keys);
+    if (keys) writeShadeKey(sc, wb, i, h.inst, keys, __activemask());
   }
   if (keys) finishShadeKeys(wb);
   if (kCount) {
@@ -342,9 +342,263 @@ __device__ __forceinline__ void persistentTraverse(const SceneView& sc, WaveBuff
       } else {
         wb.hit[ray] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
         wb.hit_inst[ray] = st.best.inst;
-        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, keys);
+        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, keys, __activemask());
       }
       ray = -1;
+    }
+  }
+  if (kCount) {
+    unsigned long long a = cnt.nodes, b = cnt.tris, c = cnt.insts;
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_down_sync(kFull, a, o);
+      b += __shfl_down_sync(kFull, b, o);
+      c += __shfl_down_sync(kFull, c, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&wb.stats[2], a);
+      atomicAdd(&wb.stats[3], b);
+      atomicAdd(&wb.stats[4], c);
+    }
+  }
+}
+
+// ---- the closest-hit and shadow walk over four-wide trees ---------------------------
+// What bounds it: the warp's lanes want different things (a node visit, the
+// triangles of a leaf, an instance entry or return, a new ray), and with one
+// resumable walk per lane a warp step ran all of them one after the other on a
+// few lanes each: 9-12 of 32 lanes active per instruction, issue slots 73 %
+// used.  Here every turn of the loop does one of three things for all lanes
+// that want it:
+//   space change  a return to the TLAS, the end of a ray, a new ray and an
+//                 instance entry; they share one computation of the slab terms
+//   leaf          the triangles of a BLAS leaf
+//   node          kNodeRuns node visits
+// The lanes vote (three ballots); a space change runs once kSpaceLanes of 32
+// active lanes want one, a leaf likewise from kLeafLanes on, and either when
+// nothing else is left, so lanes wait a little instead of running alone: 17-18
+// lanes active.  A ray's visits, tests and bounds keep their order, so hits,
+// ties included, are those of the one-ray walk.
+// The world ray, the closest hit's record and the first kWalkShort stack
+// entries are columns in shared memory (26 words a thread), which leaves the
+// registers to the node visit: 64, no spills, 32 warps an SM.  A node comes in
+// four loads (Bvh4Node).
+// Measured (closest hit, ms a frame, one pipeline, before -> after): icosphere
+// 1280x720x16 23.3 -> 17.9, instanced scene 1920x1080x8 95.8 -> 75.1, Cornell
+// room 640x480x4 (hero wavelengths) 0.83 -> 0.70; shadow rays 3.03 -> 2.70 and
+// 2.95 -> 2.70.  kSpaceLanes 6 / 8 / 10 / 14 on the instanced scene: 78.0 /
+// 75.8 / 75.1 / 75.7; kLeafLanes 6 / 8 / 10: 74.7 / 74.5 / 76.2 (icosphere
+// 18.2 / 17.9 / 18.0); kNodeRuns 1 / 2 / 3: 81.4 / 77.4 / 78.8; kWalkShort 10 /
+// 12 / 16: 75.5 / 74.9 / 74.5; 56 and 48 registers (36 and 40 warps, 44 and
+// 140 B of spills): 81.3 and 96.0; 24 warps: 81.1.
+constexpr int kSpaceLanes = 10, kLeafLanes = 8, kNodeRuns = 2;
+constexpr int kWalkShort = 16;              // stack entries per thread in shared memory
+constexpr int kWalkStack = kStackSize + 1;  // the sentinel below the stack included
+
+// Bytes of shared memory per thread: the stack column, the world ray and (kAny:
+// shadow rays have none) the closest hit.
+template <bool kAny>
+constexpr size_t walkBytes() {
+  return (kWalkShort + 6 + (kAny ? 0 : 4)) * 4;
+}
+
+// kAny: shadow rays (the first hit below a ray's bound ends it).
+template <bool kAny, bool kCount, int kNodes>
+__device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers& wb, uint32_t n,
+                                          uint32_t* work, int parity, int keys) {
+  static_assert(kNodes != kNodesBinary);
+  using W = Wide<kNodes == kNodesWide4Q>;
+  const uint32_t lane = threadIdx.x & 31u;
+  TravCounters cnt{0u, 0u, 0u};
+  extern __shared__ int32_t s_walk[];
+  const uint32_t bd = blockDim.x;
+  // columns of this thread: word k at [k * bd]
+  int32_t* const s_link = s_walk + threadIdx.x;
+  float* const s_ray = reinterpret_cast<float*>(s_walk + kWalkShort * bd) + threadIdx.x;
+  float* const s_hit = s_ray + 6 * bd;  // u, v, triangle, instance (-1: none)
+  int32_t spill[kWalkStack - kWalkShort];
+
+  float ox = 0, oy = 0, oz = 0, dx = 0, dy = 0, dz = 0;  // the ray in the current space
+  float idx = 0, idy = 0, idz = 0;                       // slab terms: t = plane * id + no
+  float nox = 0, noy = 0, noz = 0;
+  float best = 0;
+  // node: what to do next (a node, a leaf, kToTlas, kDone); cur: the instance
+  // (-1: in the TLAS); ray: the queued ray (-1: none)
+  int32_t node = kDone, sp = 0, cur = -1, ray = -1;
+  bool occluded = false, exhausted = false;
+
+  auto push = [&](int32_t link) {
+    if (sp < kWalkShort)
+      s_link[sp * bd] = link;
+    else
+      spill[sp - kWalkShort] = link;
+    ++sp;
+  };
+  auto pop = [&]() -> int32_t {  // the sentinel (kDone) ends every walk
+    --sp;
+    return sp < kWalkShort ? s_link[sp * bd] : spill[sp - kWalkShort];
+  };
+  auto overflow = [&]() {
+    atomicOr(wb.status, 1u);
+    if (!kAny) s_hit[3 * bd] = __int_as_float(-1);
+    node = kDone;
+    cur = -1;
+  };
+
+  while (true) {
+    const bool special = node < 0 && (cur < 0 || node <= kDone);
+    const unsigned at_node = __ballot_sync(kFull, node >= 0);
+    const unsigned at_leaf = __ballot_sync(kFull, node < 0 && !special);
+    const unsigned at_space = __ballot_sync(kFull, special && (ray >= 0 || !exhausted));
+    if (!(at_node | at_leaf | at_space)) break;
+    const int active = __popc(at_node | at_leaf | at_space);
+    if (at_space && (__popc(at_space) * 32 >= kSpaceLanes * active || !(at_node | at_leaf))) {
+      if (special && ray >= 0 && node == kToTlas) {
+        cur = -1;
+        node = pop();
+      }
+      const bool fin = special && ray >= 0 && node == kDone;
+      const unsigned fins = __ballot_sync(kFull, fin);
+      if (fin) {
+        if (kAny) {
+          if (!occluded) addShadowTerm(wb, static_cast<uint32_t>(ray));
+        } else {
+          const int32_t inst = __float_as_int(s_hit[3 * bd]);
+          wb.hit[ray] = make_float4(best, s_hit[0], s_hit[bd], s_hit[2 * bd]);
+          wb.hit_inst[ray] = inst;
+          if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), inst, keys, fins);
+        }
+        ray = -1;
+      }
+      const unsigned idle = __ballot_sync(kFull, ray < 0);
+      if (idle && !exhausted) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(work, static_cast<uint32_t>(__popc(idle)));
+        base = __shfl_sync(kFull, base, 0);
+        exhausted = base + static_cast<uint32_t>(__popc(idle)) >= n;
+        const uint32_t i = base + static_cast<uint32_t>(__popc(idle & ((1u << lane) - 1u)));
+        if (ray < 0 && i < n) {
+          ray = static_cast<int32_t>(i);
+          const float4 o = kAny ? wb.sh_o[i] : wb.ray_o[parity][i];
+          const float4 d = kAny ? wb.sh_d[i] : wb.ray_d[parity][i];
+          best = kAny ? fminf(d.w, MAXD) : MAXD;
+          s_ray[0] = o.x; s_ray[bd] = o.y; s_ray[2 * bd] = o.z;
+          s_ray[3 * bd] = d.x; s_ray[4 * bd] = d.y; s_ray[5 * bd] = d.z;
+          if (!kAny) {
+            s_hit[0] = 0.0f; s_hit[bd] = 0.0f; s_hit[2 * bd] = 0.0f;
+            s_hit[3 * bd] = __int_as_float(-1);
+          }
+          occluded = false;
+          sp = 0;
+          push(kDone);
+          node = 0;
+        }
+      }
+      if (special && ray >= 0) {  // the ray of the space the lane is in now
+        ox = s_ray[0]; oy = s_ray[bd]; oz = s_ray[2 * bd];
+        dx = s_ray[3 * bd]; dy = s_ray[4 * bd]; dz = s_ray[5 * bd];
+        if (node < 0 && node > kDone) {  // a TLAS leaf
+          const uint32_t first = static_cast<uint32_t>(~node) >> 3;
+          if ((static_cast<uint32_t>(~node) & 7u) == 0u) {
+            node = pop();
+          } else {
+            const float4* ipf = reinterpret_cast<const float4*>(sc.inst + first);
+            const float4 r0 = __ldg(ipf), r1 = __ldg(ipf + 1), r2 = __ldg(ipf + 2);
+            const uint4 meta = __ldg(reinterpret_cast<const uint4*>(ipf + 3));
+            const float m[12] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w};
+            if (kCount) ++cnt.insts;
+            float lx, ly, lz, ex, ey, ez;
+            toLocal(m, ox, oy, oz, dx, dy, dz, lx, ly, lz, ex, ey, ez);
+            ox = lx; oy = ly; oz = lz;
+            dx = ex; dy = ey; dz = ez;
+            cur = static_cast<int32_t>(first);
+            node = static_cast<int32_t>(meta.w);  // blas4_root
+            if (sp >= kWalkStack)
+              overflow();
+            else
+              push(kToTlas);
+          }
+        }
+        idx = safeInv(dx); idy = safeInv(dy); idz = safeInv(dz);
+        nox = -(ox * idx); noy = -(oy * idy); noz = -(oz * idz);
+      }
+    } else if (at_leaf && (__popc(at_leaf) * 32 >= kLeafLanes * active || !at_node)) {
+      if (node < 0 && !special) {
+        const uint32_t first = static_cast<uint32_t>(~node) >> 3;
+        const uint32_t count = static_cast<uint32_t>(~node) & 7u;
+        for (uint32_t k = 0; k < count; ++k) {
+          const float4* tp = sc.tris + 3u * (first + k);
+          const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+          if (kCount) ++cnt.tris;
+          float t, u, v;
+          if (intersectTri(ox, oy, oz, dx, dy, dz, ta, tb, tc, t, u, v) && t < best) {
+            if (kAny) {
+              occluded = true;
+              break;
+            }
+            best = t;
+            s_hit[0] = u;
+            s_hit[bd] = v;
+            s_hit[2 * bd] = __uint_as_float(first + k);
+            s_hit[3 * bd] = __int_as_float(cur);
+          }
+        }
+        if (kAny && occluded) {
+          node = kDone;
+          cur = -1;
+        } else {
+          node = pop();
+        }
+      }
+    } else {
+#pragma unroll
+      for (int run = 0; run < kNodeRuns; ++run) {
+        if (node < 0) continue;
+        float nxs[4], fxs[4], nys[4], fys[4], nzs[4], fzs[4];
+        const typename W::Node* nodes = cur < 0 ? W::tlas(sc) : W::blas(sc);
+        const int4 ch = W::fetch(nodes, node, idx < 0.0f, idy < 0.0f, idz < 0.0f, nxs, fxs, nys,
+                                 fys, nzs, fzs);
+        if (kCount) ++cnt.nodes;
+        float a0[4], a1[4], b0[4], b1[4], c0[4], c1[4];
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+          fma2(a0 + c, nxs + c, idx, nox);
+          fma2(a1 + c, fxs + c, idx, nox);
+          fma2(b0 + c, nys + c, idy, noy);
+          fma2(b1 + c, fys + c, idy, noy);
+          fma2(c0 + c, nzs + c, idz, noz);
+          fma2(c1 + c, fzs + c, idz, noz);
+        }
+        const int32_t links[4] = {ch.x, ch.y, ch.z, ch.w};
+        float k[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float tmin = fmaxf(fmaxf(a0[c], b0[c]), fmaxf(c0[c], 0.0f));
+          const float tmx = fminf(fminf(a1[c], b1[c]), fminf(c1[c], best));
+          const bool hit = kNodes == kNodesWide4Q ? (tmin <= tmx && links[c] != kEmptyLink)
+                                                  : tmin <= tmx;
+          k[c] = hit ? tmin : INFINITY;
+        }
+        int32_t l0 = ch.x, l1 = ch.y, l2 = ch.z, l3 = ch.w;
+        float k0 = k[0], k1 = k[1], k2 = k[2], k3 = k[3];
+        cswap(k0, l0, k1, l1);
+        cswap(k2, l2, k3, l3);
+        cswap(k0, l0, k2, l2);
+        cswap(k1, l1, k3, l3);
+        cswap(k1, l1, k2, l2);
+        if (k0 == INFINITY) {
+          node = pop();
+          continue;
+        }
+        const int pushes = (k1 != INFINITY) + (k2 != INFINITY) + (k3 != INFINITY);
+        if (sp + pushes > kWalkStack) {
+          overflow();
+          continue;
+        }
+        if (k3 != INFINITY) push(l3);
+        if (k2 != INFINITY) push(l2);
+        if (k1 != INFINITY) push(l1);
+        node = l0;
+      }
     }
   }
   if (kCount) {
@@ -381,7 +635,10 @@ __global__ void CG_EXTEND_BOUNDS k_extend_persistent(SceneView sc, WaveBuffers w
     atomicAdd(&wb.stats[0], static_cast<unsigned long long>(n));
   }
   if (keys) beginShadeKeys();
-  persistentTraverse<false, kCount, kNodes, kSpec>(sc, wb, n, &wb.counts[3], parity, keys);
+  if constexpr (kNodes == kNodesBinary || kSpec)
+    persistentTraverse<false, kCount, kNodes, kSpec>(sc, wb, n, &wb.counts[3], parity, keys);
+  else
+    walkQueue<false, kCount, kNodes>(sc, wb, n, &wb.counts[3], parity, keys);
   if (keys) finishShadeKeys(wb);
 }
 
@@ -389,7 +646,10 @@ template <bool kCount, int kNodes>
 __global__ void __launch_bounds__(256, 4) k_shadow_persistent(SceneView sc, WaveBuffers wb) {
   const uint32_t n = min(wb.counts[2], wb.capacity);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wb.stats[1], static_cast<unsigned long long>(n));
-  persistentTraverse<true, kCount, kNodes>(sc, wb, n, &wb.counts[4], 0, 0);
+  if constexpr (kNodes == kNodesBinary)
+    persistentTraverse<true, kCount, kNodes>(sc, wb, n, &wb.counts[4], 0, 0);
+  else
+    walkQueue<true, kCount, kNodes>(sc, wb, n, &wb.counts[4], 0, 0);
 }
 
 // ---- shadow: t-bounded any hit (solveEmission, trace.wesl:91-113) ----------------
@@ -1223,6 +1483,22 @@ __global__ void k_trace_closest(SceneView sc, const float4* rays, uint32_t n, fl
   }
 }
 
+// ---- row places of the four-wide nodes ----------------------------------------------
+template <class Node>
+__global__ void k_permute_rows(Node* nodes, size_t count) {
+  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  constexpr int kRows = sizeof(Node) / sizeof(uint4);
+  const uint32_t n = static_cast<uint32_t>(i);
+  const uint32_t place = kRows == 8 ? (n & 3u) << 1 : (n >> 1) & 3u;  // the walks' fetch
+  uint4* rows = reinterpret_cast<uint4*>(nodes + i);
+  uint4 in[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) in[r] = rows[r];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) rows[static_cast<uint32_t>(r) ^ place] = in[r];
+}
+
 int gSmCount = 0;
 
 uint32_t gridFor(uint32_t blocks_per_sm) {
@@ -1276,6 +1552,7 @@ void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool c
   if (ls.persistent) {  // one resident grid: 64 registers -> 65536 / (64 * block) blocks per SM
     const uint32_t g = gridFor(std::max(1u, ls.traversal_threads / block));
     const size_t smem = size_t(kShortStack) * block * sizeof(int32_t);
+    const size_t walk = walkBytes<false>() * block;
     if (ls.spec && ls.nodes != kNodesBinary) {  // postponed leaves
       const bool q = ls.nodes == kNodesWide4Q;
       if (counting) {
@@ -1290,10 +1567,10 @@ void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool c
     switch (ls.nodes * 2 + (counting ? 1 : 0)) {
       case kNodesBinary * 2: k_extend_persistent<false, kNodesBinary><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
       case kNodesBinary * 2 + 1: k_extend_persistent<true, kNodesBinary><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
-      case kNodesWide4 * 2: k_extend_persistent<false, kNodesWide4><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
-      case kNodesWide4 * 2 + 1: k_extend_persistent<true, kNodesWide4><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
-      case kNodesWide4Q * 2 + 1: k_extend_persistent<true, kNodesWide4Q><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
-      default: k_extend_persistent<false, kNodesWide4Q><<<g, block, smem, s>>>(sc, wb, parity, keys); break;
+      case kNodesWide4 * 2: k_extend_persistent<false, kNodesWide4><<<g, block, walk, s>>>(sc, wb, parity, keys); break;
+      case kNodesWide4 * 2 + 1: k_extend_persistent<true, kNodesWide4><<<g, block, walk, s>>>(sc, wb, parity, keys); break;
+      case kNodesWide4Q * 2 + 1: k_extend_persistent<true, kNodesWide4Q><<<g, block, walk, s>>>(sc, wb, parity, keys); break;
+      default: k_extend_persistent<false, kNodesWide4Q><<<g, block, walk, s>>>(sc, wb, parity, keys); break;
     }
     return;
   }
@@ -1369,13 +1646,14 @@ void launchShadow(const SceneView& sc, const WaveBuffers& wb, bool counting,
   const uint32_t block = ls.extend_block;
   if (ls.persistent) {
     const uint32_t g = gridFor(std::max(1u, ls.traversal_threads / block));
+    const size_t walk = walkBytes<true>() * block;
     switch (ls.nodes * 2 + (counting ? 1 : 0)) {
       case kNodesBinary * 2: k_shadow_persistent<false, kNodesBinary><<<g, block, 0, s>>>(sc, wb); break;
       case kNodesBinary * 2 + 1: k_shadow_persistent<true, kNodesBinary><<<g, block, 0, s>>>(sc, wb); break;
-      case kNodesWide4 * 2: k_shadow_persistent<false, kNodesWide4><<<g, block, 0, s>>>(sc, wb); break;
-      case kNodesWide4 * 2 + 1: k_shadow_persistent<true, kNodesWide4><<<g, block, 0, s>>>(sc, wb); break;
-      case kNodesWide4Q * 2 + 1: k_shadow_persistent<true, kNodesWide4Q><<<g, block, 0, s>>>(sc, wb); break;
-      default: k_shadow_persistent<false, kNodesWide4Q><<<g, block, 0, s>>>(sc, wb); break;
+      case kNodesWide4 * 2: k_shadow_persistent<false, kNodesWide4><<<g, block, walk, s>>>(sc, wb); break;
+      case kNodesWide4 * 2 + 1: k_shadow_persistent<true, kNodesWide4><<<g, block, walk, s>>>(sc, wb); break;
+      case kNodesWide4Q * 2 + 1: k_shadow_persistent<true, kNodesWide4Q><<<g, block, walk, s>>>(sc, wb); break;
+      default: k_shadow_persistent<false, kNodesWide4Q><<<g, block, walk, s>>>(sc, wb); break;
     }
     return;
   }
@@ -1433,6 +1711,14 @@ __global__ void k_film_rgba8(const float4* __restrict__ film, uchar4* __restrict
 void launchFilmRgba8(const float4* film, uchar4* rgba, size_t npx, cudaStream_t s) {
   if (npx == 0) return;
   k_film_rgba8<<<static_cast<unsigned>((npx + 255) / 256), 256, 0, s>>>(film, rgba, npx);
+}
+
+void launchPermuteNodes(Bvh4Node* nodes, size_t count, cudaStream_t s) {
+  if (count) k_permute_rows<<<static_cast<unsigned>((count + 255) / 256), 256, 0, s>>>(nodes, count);
+}
+
+void launchPermuteNodes(Bvh4QNode* nodes, size_t count, cudaStream_t s) {
+  if (count) k_permute_rows<<<static_cast<unsigned>((count + 255) / 256), 256, 0, s>>>(nodes, count);
 }
 
 void launchFilmPack(const float4* film, float* out, size_t npx, bool rgb, cudaStream_t s) {

@@ -144,6 +144,11 @@ void launchFilmRgba8(const float4* film, uchar4* rgba, size_t npx, cudaStream_t 
 void launchTraceClosest(const SceneView& sc, const float4* rays, uint32_t n, float4* out_tuv,
                         int4* out_ids, uint32_t* status, int nodes, cudaStream_t s);
 
+// Permutes the rows inside every four-wide node to their places on the device
+// (Bvh4Node, Bvh4QNode), once after the upload.
+void launchPermuteNodes(Bvh4Node* nodes, size_t count, cudaStream_t s);
+void launchPermuteNodes(Bvh4QNode* nodes, size_t count, cudaStream_t s);
+
 int smCount();
 // Sets kernel attributes on the current device (once per device, outside any
 // stream capture).

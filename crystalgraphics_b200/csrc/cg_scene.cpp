@@ -294,8 +294,7 @@ int packScene(const cg_scene_desc* d, HostScene& s, std::string& err) {
 
   // ---- one BLAS per mesh ------------------------------------------------------
   s.mesh_count = d->mesh_count;
-  std::vector<uint32_t> mesh_root(d->mesh_count), mesh_root4(d->mesh_count),
-      mesh_tri_base(d->mesh_count);
+  std::vector<uint32_t> mesh_root(d->mesh_count), mesh_root4(d->mesh_count);
   std::vector<Box> mesh_bounds(d->mesh_count);
   BvhBuildOptions blas_opt;
   blas_opt.max_leaf = 4;
@@ -328,7 +327,6 @@ int packScene(const cg_scene_desc* d, HostScene& s, std::string& err) {
     }
     mesh_bounds[m] = mb;
     const uint32_t tri_base = static_cast<uint32_t>(s.tri_vidx.size() / 4);
-    mesh_tri_base[m] = tri_base;
     order.clear();
     uint32_t depth = 0;
     mesh_root[m] = buildBvh(boxes, blas_opt, tri_base, s.blas, order, &depth);
@@ -410,7 +408,7 @@ int packScene(const cg_scene_desc* d, HostScene& s, std::string& err) {
     invertAffine(ci.world_from_local, di.inv);
     di.blas_root = mesh_root[ci.mesh];
     di.material = ci.material;
-    di.tri_base = mesh_tri_base[ci.mesh];
+    di.kind = (s.mat[ci.material].volume >> kKindShift) & 15u;
     di.blas4_root = mesh_root4[ci.mesh];
     s.inst.push_back(di);
     // world box: the corners of the mesh's BVH cut boxes, transformed in

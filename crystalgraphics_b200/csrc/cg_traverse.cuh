@@ -209,6 +209,21 @@ __device__ __forceinline__ float byteToFloat(uint32_t w, uint32_t c) {
   return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | c)) - 8388608.0f;
 }
 
+// d[0..1] = fmaf(a[0..1], b, c): two fused multiply-adds in one instruction.
+__device__ __forceinline__ void fma2(float* d, const float* a, float b, float c) {
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\t"
+      "mov.b64 c, {%5, %5};\n\tfma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d[0]), "=f"(d[1])
+      : "f"(a[0]), "f"(a[1]), "f"(b), "f"(c));
+}
+
+// 32 bytes in one load (p 32-byte aligned, read-only data).
+__device__ __forceinline__ void ldg256(const void* p, uint32_t w[8]) {
+  asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+        "=r"(w[7])
+      : "l"(p));
+}
 // The two four-wide node formats: full-precision child slabs, or 8-bit
 // offsets from the node origin (decoded to world-space bounds that contain
 // the full-precision ones: fmaf rounds q * scale + origin to nearest, and the
@@ -226,21 +241,27 @@ struct Wide<false> {
   using Node = Bvh4Node;
   static __device__ __forceinline__ const Node* tlas(const SceneView& sc) { return sc.tlas4; }
   static __device__ __forceinline__ const Node* blas(const SceneView& sc) { return sc.blas4; }
-  static __device__ __forceinline__ int4 fetch(const Node* n, bool negx, bool negy, bool negz,
-                                               float nx[4], float fx[4], float ny[4], float fy[4],
-                                               float nz[4], float fz[4]) {
-    const float4* np = reinterpret_cast<const float4*>(n);
-    // float4 rows: lo.x, hi.x, lo.y, hi.y, lo.z, hi.z
-    const float4 a = __ldg(np + (negx ? 1 : 0)), b = __ldg(np + (negx ? 0 : 1));
-    const float4 c = __ldg(np + (negy ? 3 : 2)), d = __ldg(np + (negy ? 2 : 3));
-    const float4 e = __ldg(np + (negz ? 5 : 4)), f = __ldg(np + (negz ? 4 : 5));
-    nx[0] = a.x; nx[1] = a.y; nx[2] = a.z; nx[3] = a.w;
-    fx[0] = b.x; fx[1] = b.y; fx[2] = b.z; fx[3] = b.w;
-    ny[0] = c.x; ny[1] = c.y; ny[2] = c.z; ny[3] = c.w;
-    fy[0] = d.x; fy[1] = d.y; fy[2] = d.z; fy[3] = d.w;
-    nz[0] = e.x; nz[1] = e.y; nz[2] = e.z; nz[3] = e.w;
-    fz[0] = f.x; fz[1] = f.y; fz[2] = f.z; fz[3] = f.w;
-    return __ldg(reinterpret_cast<const int4*>(np + 6));
+  static __device__ __forceinline__ int4 fetch(const Node* nodes, int32_t n, bool negx, bool negy,
+                                               bool negz, float nx[4], float fx[4], float ny[4],
+                                               float fy[4], float nz[4], float fz[4]) {
+    const char* np = reinterpret_cast<const char*>(nodes + n);
+    // row pair p (lo and hi of an axis, or the links) is at place p ^ (n & 3)
+    const uint32_t sw = (static_cast<uint32_t>(n) & 3u) << 5;
+    uint32_t x[8], y[8], z[8];
+    ldg256(np + sw, x);
+    ldg256(np + (sw ^ 32u), y);
+    ldg256(np + (sw ^ 64u), z);
+    const int4 links = __ldg(reinterpret_cast<const int4*>(np + (sw ^ 96u)));
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      nx[c] = __uint_as_float(negx ? x[4 + c] : x[c]);
+      fx[c] = __uint_as_float(negx ? x[c] : x[4 + c]);
+      ny[c] = __uint_as_float(negy ? y[4 + c] : y[c]);
+      fy[c] = __uint_as_float(negy ? y[c] : y[4 + c]);
+      nz[c] = __uint_as_float(negz ? z[4 + c] : z[c]);
+      fz[c] = __uint_as_float(negz ? z[c] : z[4 + c]);
+    }
+    return links;
   }
 };
 
@@ -249,13 +270,14 @@ struct Wide<true> {
   using Node = Bvh4QNode;
   static __device__ __forceinline__ const Node* tlas(const SceneView& sc) { return sc.tlas4q; }
   static __device__ __forceinline__ const Node* blas(const SceneView& sc) { return sc.blas4q; }
-  static __device__ __forceinline__ int4 fetch(const Node* n, bool negx, bool negy, bool negz,
-                                               float nx[4], float fx[4], float ny[4], float fy[4],
-                                               float nz[4], float fz[4]) {
-    const float4* np = reinterpret_cast<const float4*>(n);
-    const float4 h = __ldg(np);
-    const uint4 qa = __ldg(reinterpret_cast<const uint4*>(np + 1));  // lo.x hi.x lo.y hi.y
-    const uint4 qb = __ldg(reinterpret_cast<const uint4*>(np + 2));  // lo.z hi.z
+  static __device__ __forceinline__ int4 fetch(const Node* nodes, int32_t n, bool negx, bool negy,
+                                               bool negz, float nx[4], float fx[4], float ny[4],
+                                               float fy[4], float nz[4], float fz[4]) {
+    const float4* np = reinterpret_cast<const float4*>(nodes + n);
+    const uint32_t sw = (static_cast<uint32_t>(n) >> 1) & 3u;  // row r at slot r ^ sw
+    const float4 h = __ldg(np + sw);
+    const uint4 qa = __ldg(reinterpret_cast<const uint4*>(np + (sw ^ 1u)));  // lo.x hi.x lo.y hi.y
+    const uint4 qb = __ldg(reinterpret_cast<const uint4*>(np + (sw ^ 2u)));  // lo.z hi.z
     const uint32_t sb = __float_as_uint(h.w);
     const float sx = __uint_as_float((sb & 0xffu) << 23);
     const float sy = __uint_as_float(((sb >> 8) & 0xffu) << 23);
@@ -272,7 +294,7 @@ struct Wide<true> {
       nz[c] = fmaf(byteToFloat(wnz, c), sz, h.z);
       fz[c] = fmaf(byteToFloat(wfz, c), sz, h.z);
     }
-    return __ldg(reinterpret_cast<const int4*>(np + 3));
+    return __ldg(reinterpret_cast<const int4*>(np + (sw ^ 3u)));
   }
 };
 
@@ -349,7 +371,7 @@ __device__ __forceinline__ bool travSteps(const SceneView& sc, TravState& s, Sta
       using W = Wide<kNodes == kNodesWide4Q>;
       const typename W::Node* nodes = s.cur_inst < 0 ? W::tlas(sc) : W::blas(sc);
       float nxs[4], fxs[4], nys[4], fys[4], nzs[4], fzs[4];
-      const int4 ch = W::fetch(nodes + node, s.idx < 0.0f, s.idy < 0.0f, s.idz < 0.0f, nxs, fxs,
+      const int4 ch = W::fetch(nodes, node, s.idx < 0.0f, s.idy < 0.0f, s.idz < 0.0f, nxs, fxs,
                                nys, fys, nzs, fzs);
       if (kCount) ++cnt.nodes;
       float k[4];
@@ -516,7 +538,7 @@ __device__ __forceinline__ bool travStepsSpec(const SceneView& sc, TravState& s,
       if (node >= 0) {  // one inner node visit
         const typename W::Node* nodes = s.cur_inst < 0 ? W::tlas(sc) : W::blas(sc);
         float nxs[4], fxs[4], nys[4], fys[4], nzs[4], fzs[4];
-        const int4 ch = W::fetch(nodes + node, s.idx < 0.0f, s.idy < 0.0f, s.idz < 0.0f, nxs, fxs,
+        const int4 ch = W::fetch(nodes, node, s.idx < 0.0f, s.idy < 0.0f, s.idz < 0.0f, nxs, fxs,
                                  nys, fys, nzs, fzs);
         if (kCount) ++cnt.nodes;
         float k[4];
@@ -647,7 +669,7 @@ __device__ __forceinline__ HitRec traceRay4(const SceneView& sc, float wox, floa
   while (true) {
     while (node >= 0) {
       float nxs[4], fxs[4], nys[4], fys[4], nzs[4], fzs[4];
-      const int4 ch = W::fetch(nodes + node, idx < 0.0f, idy < 0.0f, idz < 0.0f, nxs, fxs, nys, fys,
+      const int4 ch = W::fetch(nodes, node, idx < 0.0f, idy < 0.0f, idz < 0.0f, nxs, fxs, nys, fys,
                                nzs, fzs);
       if (kCount) ++cnt.nodes;
       float k[4];
