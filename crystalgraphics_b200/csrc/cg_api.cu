@@ -557,8 +557,10 @@ int Renderer::enqueueViews(const SceneDev& scene, const std::vector<ViewDev>& vi
     CG_CUDA(cudaEventRecord(fork_ev, s));
     for (int k = 0; k + 1 < P; ++k) CG_CUDA(cudaStreamWaitEvent(xstream[k], fork_ev, 0));
   }
+  rec.pipelines = static_cast<uint32_t>(P);
   for (size_t k = 0; k < chunks.size(); ++k) {
     const int p = static_cast<int>(k % static_cast<size_t>(P));
+    chunks[k].reset = k < static_cast<size_t>(P) ? 1u : 0u;
     enqueueChunk(scene, static_cast<uint32_t>(views.size()), table, chunks[k], caps,
                  p ? xstream[p - 1] : s, rec, p ? &xwave[p - 1] : &wave);
   }
@@ -601,54 +603,40 @@ void Renderer::profCollect() {
   prof_used = 0;
 }
 
-int Renderer::beginStats(cudaStream_t s) {
-  CG_CUDA(cudaMemsetAsync(wave.stats, 0, 256, s));
-  CG_CUDA(cudaMemsetAsync(wave.status, 0, 256, s));
-  for (int k = 0; k < kMaxPipelines - 1; ++k)
-    if (xwave_arena[k].base) {  // ordered before the fork the extra pipelines wait on
-      CG_CUDA(cudaMemsetAsync(xwave[k].stats, 0, 256, s));
-      CG_CUDA(cudaMemsetAsync(xwave[k].status, 0, 256, s));
-    }
+int Renderer::fetchStats(cudaStream_t s, const RenderRecord& rec) {
+  for (uint32_t p = 0; p < rec.pipelines; ++p) {
+    const WaveBuffers& w = p ? xwave[p - 1] : wave;
+    CG_CUDA(cudaMemcpyAsync(stats_host + p * kStatsHostStride, w.stats, kStatusAt + 4,
+                            cudaMemcpyDeviceToHost, s));
+  }
   return CG_OK;
 }
 
-int Renderer::readStats(cudaStream_t s, const RenderRecord& rec, float ms, cg_stats& out) {
-  unsigned long long st[kMaxPipelines][8] = {};
-  uint32_t status[kMaxPipelines] = {};
-  bool used[kMaxPipelines] = {true};
-  for (int k = 0; k < kMaxPipelines - 1; ++k)
-    used[k + 1] = xwave_arena[k].base != nullptr;  // zeroed by beginStats; read after the join
-  for (int p = 0; p < kMaxPipelines; ++p) {
-    if (!used[p]) continue;
-    const WaveBuffers& w = p ? xwave[p - 1] : wave;
-    unsigned char* h = stats_host + p * kStatsHostStride;
-    CG_CUDA(cudaMemcpyAsync(h, w.stats, sizeof(st[0]), cudaMemcpyDeviceToHost, s));
-    CG_CUDA(cudaMemcpyAsync(h + sizeof(st[0]), w.status, 4, cudaMemcpyDeviceToHost, s));
-  }
-  CG_CUDA(cudaStreamSynchronize(s));
-  for (int p = 0; p < kMaxPipelines; ++p) {
-    if (!used[p]) continue;
+int Renderer::readStats(const RenderRecord& rec, float ms, cg_stats& out) {
+  unsigned long long st[kStatWords] = {};
+  uint32_t status = 0;
+  for (uint32_t p = 0; p < rec.pipelines; ++p) {
     const unsigned char* h = stats_host + p * kStatsHostStride;
-    std::memcpy(st[p], h, sizeof(st[0]));
-    std::memcpy(&status[p], h + sizeof(st[0]), 4);
-  }
-  for (int p = 1; p < kMaxPipelines; ++p) {
-    for (int k = 0; k < 8; ++k) st[0][k] += st[p][k];
-    status[0] |= status[p];
+    unsigned long long x[kStatWords];
+    uint32_t bits;
+    std::memcpy(x, h, sizeof(x));
+    std::memcpy(&bits, h + kStatusAt, 4);
+    for (int k = 0; k < kStatWords; ++k) st[k] += x[k];
+    status |= bits;
   }
   profCollect();
   out.samples = rec.samples;
-  out.extend_rays = st[0][0];
-  out.shadow_rays = st[0][1];
-  out.node_visits = st[0][2];
-  out.tri_tests = st[0][3];
-  out.inst_visits = st[0][4];
-  out.nonfinite_samples = st[0][5];
+  out.extend_rays = st[0];
+  out.shadow_rays = st[1];
+  out.node_visits = st[2];
+  out.tri_tests = st[3];
+  out.inst_visits = st[4];
+  out.nonfinite_samples = st[5];
   out.chunks = rec.chunks;
   out.kernel_launches = rec.launches;
   out.device_ms = ms;
-  if (status[0] & 1u) return fail(CG_E_DEVICE, "traversal stack overflow in a kernel");
-  if (status[0] & 2u) return fail(CG_E_DEVICE, "ray queue overflow in a kernel");
+  if (status & 1u) return fail(CG_E_DEVICE, "traversal stack overflow in a kernel");
+  if (status & 2u) return fail(CG_E_DEVICE, "ray queue overflow in a kernel");
   return CG_OK;
 }
 
@@ -656,24 +644,12 @@ int Renderer::readStats(cudaStream_t s, const RenderRecord& rec, float ms, cg_st
 Env* g_env = nullptr;
 std::mutex g_env_mu;
 
-int Env::uploadViews(const std::vector<ViewDev>& views, cudaStream_t s) {
-  if (views.size() > view_cap) {
-    if (views_dev) cudaFree(views_dev);
-    views_dev = nullptr;
-    view_cap = 0;
-    CG_CUDA(cudaMalloc(&views_dev, views.size() * sizeof(ViewDev)));
-    view_cap = views.size();
-  }
-  CG_CUDA(cudaMemcpyAsync(views_dev, views.data(), views.size() * sizeof(ViewDev),
-                          cudaMemcpyHostToDevice, s));
-  return CG_OK;
-}
-
 Env::~Env() {
   if (stream) cudaStreamSynchronize(stream);
   graphs.clear();
-  dropViewGraph();
+  dropViewGraphs();
   if (views_dev) cudaFree(views_dev);
+  if (view_host) cudaFreeHost(view_host);
   if (film) cudaFree(film);
   if (rgba) cudaFree(rgba);
   if (film_pack) cudaFree(film_pack);
@@ -710,15 +686,23 @@ static int createEnv(const cg_conf& conf_in, int device, std::unique_ptr<Env>& o
   CG_CUDA(cudaMalloc(&env->film, npx * sizeof(float4)));
   CG_CUDA(cudaMalloc(&env->rgba, npx * sizeof(uchar4)));
   CG_CUDA(cudaMalloc(&env->film_pack, npx * 3 * sizeof(float)));
+  CG_CUDA(cudaMalloc(&env->views_dev, sizeof(ViewDev)));
+  CG_CUDA(cudaMallocHost(&env->view_host, sizeof(ViewDev)));
   CG_CUDA(cudaMemset(env->film, 0, npx * sizeof(float4)));
   CG_CUDA(cudaMemset(env->rgba, 0, npx * sizeof(uchar4)));
   out = std::move(env);
   return CG_OK;
 }
 
-// Renders one prepared view of `s` into the environment's film: uploads the
-// view table and enqueues (or, when `allow_graph`, replays the captured)
-// launch sequence, then waits and reads the statistics.
+// Renders one prepared view of `s` into the environment's film: the view's
+// copy to the device, the launch sequence, the copies of the statistics and
+// one wait.  With `allow_graph` a scene's second frame captures all of it as
+// one graph and later frames replay it (Env::ViewGraph): it depends only on
+// the scene, the conf, the tuning and the buffers, and the view changes in
+// pinned memory.  Small frames are bound by this host path: as memsets, a
+// pageable copy, one graph kept for the scene viewed last, its events, four
+// copies and two waits, a 256x256 frame of the Cornell room took 175 us (133 on
+// the device), and 329 us with scenes taking turns; now 150 and 155.
 static int renderEnvView(Env& env, SceneDev* s, std::vector<ViewDev>& views, bool allow_graph) {
   layoutViews(views);
   const Caps caps = capsOf(env.conf);
@@ -729,55 +713,50 @@ static int renderEnvView(Env& env, SceneDev* s, std::vector<ViewDev>& views, boo
     rc = env.ensurePipelines(static_cast<int>(env.tuning.pipelines));
     if (rc != CG_OK) return rc;
   }
-  rc = env.beginStats(env.stream);
-  if (rc != CG_OK) return rc;
-  rc = env.uploadViews(views, env.stream);
-  if (rc != CG_OK) return rc;
-  const ViewDev* table = static_cast<const ViewDev*>(env.views_dev);
+  *env.view_host = views[0];  // every earlier copy from it has been waited for
+  auto enqueue = [&](RenderRecord& rec, unsigned event_flags) -> int {
+    CG_CUDA(cudaMemcpyAsync(env.views_dev, env.view_host, sizeof(ViewDev), cudaMemcpyHostToDevice,
+                            env.stream));
+    CG_CUDA(cudaEventRecordWithFlags(env.ev0, env.stream, event_flags));
+    const int e = env.enqueueViews(*s, views, static_cast<const ViewDev*>(env.views_dev), caps,
+                                   env.stream, rec);
+    if (e != CG_OK) return e;
+    CG_CUDA(cudaEventRecordWithFlags(env.ev1, env.stream, event_flags));
+    return env.fetchStats(env.stream, rec);
+  };
   RenderRecord rec;
-  if (use_graph) {
-    // the launch sequence depends only on the scene, the conf, the tuning and
-    // the buffers, so it is captured once and replayed: a small frame's ~60
-    // launches then cost one graph launch
-    Env::ViewGraph& vg = env.view_graph;
-    if (!(vg.exec && vg.scene_tag == s->tag && vg.counting == env.counting && vg.table == table)) {
-      env.dropViewGraph();
-      CG_CUDA(cudaStreamSynchronize(env.stream));
+  Env::ViewGraph* vg = use_graph ? env.viewGraphOf(s->tag) : nullptr;
+  if (vg) {
+    if (!vg->exec) {
       cudaGraph_t graph = nullptr;
       CG_CUDA(cudaStreamBeginCapture(env.stream, cudaStreamCaptureModeThreadLocal));
       RenderRecord r;
-      rc = env.enqueueViews(*s, views, table, caps, env.stream, r);
+      rc = enqueue(r, cudaEventRecordExternal);
       cudaError_t ce = cudaStreamEndCapture(env.stream, &graph);
       if (rc != CG_OK) {
         if (graph) cudaGraphDestroy(graph);
         return rc;
       }
       if (ce != cudaSuccess) return cudaFail(ce, "cudaStreamEndCapture");
-      ce = cudaGraphInstantiate(&vg.exec, graph, 0);
+      ce = cudaGraphInstantiate(&vg->exec, graph, 0);
       cudaGraphDestroy(graph);
       if (ce != cudaSuccess) {
-        vg.exec = nullptr;
+        vg->exec = nullptr;
         return cudaFail(ce, "cudaGraphInstantiate");
       }
-      vg.scene_tag = s->tag;
-      vg.counting = env.counting;
-      vg.table = table;
-      vg.rec = r;
+      vg->rec = r;
     }
-    CG_CUDA(cudaEventRecord(env.ev0, env.stream));
-    CG_CUDA(cudaGraphLaunch(vg.exec, env.stream));
-    rec = vg.rec;
+    CG_CUDA(cudaGraphLaunch(vg->exec, env.stream));
+    rec = vg->rec;
   } else {
-    CG_CUDA(cudaEventRecord(env.ev0, env.stream));
-    rc = env.enqueueViews(*s, views, table, caps, env.stream, rec);
+    rc = enqueue(rec, cudaEventRecordDefault);
     if (rc != CG_OK) return rc;
   }
-  CG_CUDA(cudaEventRecord(env.ev1, env.stream));
   CG_CUDA(cudaGetLastError());
-  CG_CUDA(cudaEventSynchronize(env.ev1));
+  CG_CUDA(cudaStreamSynchronize(env.stream));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, env.ev0, env.ev1);
-  return env.endStats(env.stream, rec, ms);
+  return env.readStats(rec, ms, env.last);
 }
 
 }  // namespace cg
@@ -1106,7 +1085,11 @@ CG_API int cg_film_read(void* host, size_t bytes, int format) {
     Env& env = *g_env;
     const size_t npx = size_t(env.conf.render_width) * env.conf.render_height;
     CG_CUDA(cudaSetDevice(env.device));
-    prefaultHostBuffer(host, std::min(bytes, npx * (format == CG_FILM_RGBA8 ? 4 : 12)));
+    // (a pinned buffer is mapped already)
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) cudaGetLastError();
+    if (attr.type != cudaMemoryTypeHost)
+      prefaultHostBuffer(host, std::min(bytes, npx * (format == CG_FILM_RGBA8 ? 4 : 12)));
     if (format == CG_FILM_RGBA8) {
       if (bytes < npx * 4) return fail(CG_E_INVALID, "buffer too small for RGBA8");
       CG_CUDA(cudaMemcpyAsync(host, env.rgba, npx * 4, cudaMemcpyDeviceToHost, env.stream));
@@ -1198,7 +1181,7 @@ CG_API int cg_set_spectral(int mode) {
     CG_CUDA(cudaSetDevice(env.device));
     CG_CUDA(cudaStreamSynchronize(env.stream));
     env.dropAllGraphs();  // captured launch sequences use the other mode's kernels
-    env.dropViewGraph();
+    env.dropViewGraphs();
     env.spectral = mode;
     env.hero = mode == CG_SPECTRAL_HERO;
     env.has_prev = false;  // the film's running mean restarts
@@ -1216,7 +1199,7 @@ CG_API int cg_set_roulette(uint32_t start_depth) {
     CG_CUDA(cudaSetDevice(env.device));
     CG_CUDA(cudaStreamSynchronize(env.stream));
     env.dropAllGraphs();  // captured launches hold the old setting
-    env.dropViewGraph();
+    env.dropViewGraphs();
     env.roulette = start_depth;
     env.has_prev = false;  // the film's running mean restarts
     return CG_OK;

@@ -110,6 +110,7 @@ struct RenderRecord {
   uint64_t samples = 0;
   uint32_t chunks = 0;
   uint32_t launches = 0;
+  uint32_t pipelines = 1;  // queue sets the chunks ran on
 };
 
 // Device resources of one launch stream: wavelength tables, ray queues and
@@ -120,9 +121,10 @@ struct Renderer {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float* wl_tree = nullptr;
   float* wl_const = nullptr;
-  // pinned: each pipeline's statistics (64 B) and status word, read back
-  // with asynchronous copies and one synchronisation
-  static constexpr size_t kStatsHostStride = 128;
+  // pinned: each pipeline's statistics and status word (one copy of the 260
+  // bytes that hold both), read back with one synchronisation
+  static constexpr size_t kStatsHostStride = 512;
+  static constexpr size_t kStatusAt = 256;  // the status word behind the statistics (allocWave)
   unsigned char* stats_host = nullptr;
   bool counting = false;
   // 64M rays per level queue (~11.1 GB of path state): large chunks keep every
@@ -170,8 +172,11 @@ struct Renderer {
   void enqueueChunk(const SceneDev& scene, uint32_t view_count, const ViewDev* table,
                     const ChunkDesc& ch, const Caps& caps, cudaStream_t s, RenderRecord& rec,
                     const WaveBuffers* wbp = nullptr);
-  int beginStats(cudaStream_t s);
-  int readStats(cudaStream_t s, const RenderRecord& rec, float ms, cg_stats& out);
+  // Statistics of a run: the first chunk of every queue set zeroes them
+  // (ChunkDesc::reset), fetchStats enqueues their copies behind the run, and
+  // readStats sums them once the stream has been synchronised.
+  int fetchStats(cudaStream_t s, const RenderRecord& rec);
+  int readStats(const RenderRecord& rec, float ms, cg_stats& out);
 
   // Per-kernel CUDA-event timing (off by default; never inside a capture).
   bool profiling = false;
@@ -215,26 +220,28 @@ struct Env : Renderer {
   uint32_t frame_count = 0;
   uint32_t seed = 0;
   void* views_dev = nullptr;
-  size_t view_cap = 0;
+  ViewDev* view_host = nullptr;  // pinned: the one view of cg_view and cg_view_samples
   cg_stats last{};
   std::vector<std::unique_ptr<BatchGraph>> graphs;
-  // View()'s launch sequence, captured once per scene and replayed (the view
-  // table it reads is uploaded before every replay); valid while the scene,
-  // the counting mode and the table's address are the ones it was captured
-  // with (tuning changes drop it)
+  // View()'s run as a captured graph, one per scene: the copy of the view from
+  // pinned memory, the launch sequence between ev0 and ev1, and the copies of
+  // the statistics.  The first frame of a scene is launched directly (capturing
+  // and instantiating takes longer than the launches save there), the second
+  // one captures, later ones replay.  The kMaxViewGraphs scenes viewed last
+  // keep theirs; a tuning change drops all, a destroyed scene its own.
+  static constexpr size_t kMaxViewGraphs = 8;
   struct ViewGraph {
     uint64_t scene_tag = 0;
     bool counting = false;
-    const void* table = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec = nullptr;  // null: the scene has had its first frame
     RenderRecord rec;
-  } view_graph;
-  void dropViewGraph();
+  };
+  std::vector<ViewGraph> view_graphs;  // most recently used last
+  // The entry of a scene in the current counting mode, moved to the back; null
+  // where there was none (an entry without a graph is added then)
+  ViewGraph* viewGraphOf(uint64_t scene_tag);
+  void dropViewGraphs();
 
-  int uploadViews(const std::vector<ViewDev>& views, cudaStream_t s);
-  int endStats(cudaStream_t s, const RenderRecord& rec, float ms) {
-    return readStats(s, rec, ms, last);
-  }
   void dropGraphsFor(uint64_t tag);
   void dropAllGraphs();
   ~Env();

@@ -27,15 +27,37 @@ void Env::dropGraphsFor(uint64_t tag) {
   graphs.erase(std::remove_if(graphs.begin(), graphs.end(),
                               [&](const std::unique_ptr<BatchGraph>& g) { return g->scene_tag == tag; }),
                graphs.end());
-  if (view_graph.exec && view_graph.scene_tag == tag) dropViewGraph();
+  for (size_t k = view_graphs.size(); k-- > 0;)
+    if (view_graphs[k].scene_tag == tag) {
+      if (view_graphs[k].exec) cudaGraphExecDestroy(view_graphs[k].exec);
+      view_graphs.erase(view_graphs.begin() + static_cast<ptrdiff_t>(k));
+    }
 }
 void Env::dropAllGraphs() {
   graphs.clear();
-  dropViewGraph();
+  dropViewGraphs();
 }
-void Env::dropViewGraph() {
-  if (view_graph.exec) cudaGraphExecDestroy(view_graph.exec);
-  view_graph = ViewGraph{};
+void Env::dropViewGraphs() {
+  for (ViewGraph& g : view_graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  view_graphs.clear();
+}
+Env::ViewGraph* Env::viewGraphOf(uint64_t scene_tag) {
+  for (size_t k = 0; k < view_graphs.size(); ++k)
+    if (view_graphs[k].scene_tag == scene_tag && view_graphs[k].counting == counting) {
+      std::rotate(view_graphs.begin() + static_cast<ptrdiff_t>(k),
+                  view_graphs.begin() + static_cast<ptrdiff_t>(k) + 1, view_graphs.end());
+      return &view_graphs.back();
+    }
+  if (view_graphs.size() >= kMaxViewGraphs) {
+    if (view_graphs.front().exec) cudaGraphExecDestroy(view_graphs.front().exec);
+    view_graphs.erase(view_graphs.begin());
+  }
+  ViewGraph g;
+  g.scene_tag = scene_tag;
+  g.counting = counting;
+  view_graphs.push_back(g);
+  return nullptr;
 }
 
 // Builds the view table of a batch into `g` (films allocated per view).
@@ -170,14 +192,15 @@ CG_API int cg_batch_render(cg_scene_t scene, const cg_view_desc* views, uint32_t
     CG_CUDA(cudaSetDevice(env.device));
     int rc = env.ensureWave(env.tuning.queue_capacity);
     if (rc != CG_OK) return rc;
-    rc = env.beginStats(env.stream);
-    if (rc != CG_OK) return rc;
     BatchGraph* g = nullptr;
     RenderRecord rec;
     float ms = 0.0f;
     rc = runBatch(env, *s, views, view_count, g, rec, ms);
     if (rc != CG_OK) return rc;
-    rc = env.endStats(env.stream, rec, ms);
+    rc = env.fetchStats(env.stream, rec);
+    if (rc != CG_OK) return rc;
+    CG_CUDA(cudaStreamSynchronize(env.stream));
+    rc = env.readStats(rec, ms, env.last);
     if (rc != CG_OK) return rc;
     // readback
     const char* base = static_cast<const char*>(g->films.base);

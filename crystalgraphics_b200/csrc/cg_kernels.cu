@@ -93,6 +93,10 @@ __global__ void k_gen(FrameConst fc, WaveBuffers wb, ChunkDesc ch) {
     wb.counts[2] = 0u;
     wb.counts[3] = 0u;  // work counters of the persistent traversal
     wb.counts[4] = 0u;
+    if (ch.reset) {
+      for (int k = 0; k < kStatWords; ++k) wb.stats[k] = 0ull;
+      *wb.status = 0u;
+    }
   }
   if (i >= ch.sample_count) return;
   const uint64_t g = ch.sample_begin + i;

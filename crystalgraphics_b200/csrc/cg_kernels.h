@@ -40,6 +40,8 @@ struct Caps {
   uint32_t trace_depth, transport_cap, emission_cap, diffuse_cap, rough_cap;
 };
 
+constexpr int kStatWords = 8;  // 64-bit statistics of a queue set (WaveBuffers::stats)
+
 // Wavefront buffers (device).
 struct WaveBuffers {
   float4* ray_o[2];      // origin.xyz, path weight
@@ -99,6 +101,7 @@ struct ChunkDesc {
   uint64_t pixel_begin;
   uint32_t sample_count;
   uint32_t pixel_count;
+  uint32_t reset = 0;  // the first chunk of its queue set in a run: zeroes its statistics and status
 };
 
 // How the shading kernel orders a level's rays: as queued, by a counting
