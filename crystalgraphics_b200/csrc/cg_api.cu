@@ -175,6 +175,7 @@ int uploadScene(const HostScene& h, SceneDev& s) {
   v.env_h = h.env_h;
   v.emissive_count = static_cast<uint32_t>(h.eprim.size());
   v.instance_count = static_cast<uint32_t>(h.inst.size());
+  v.nodes4 = static_cast<uint32_t>(h.blas4.size() + h.tlas4.size());
   v.has_tlas = h.inst.empty() ? 0u : 1u;
   v.has_lights = h.eprim.empty() ? 0u : 1u;
   s.eprim_off = parts[7].off;
@@ -470,6 +471,7 @@ void Renderer::enqueueChunk(const SceneDev& scene, uint32_t view_count, const Vi
   ls.persistent = tuning.persistent != 2u;
   ls.spec = tuning.persistent == 3u;
   ls.traversal_threads = tuning.traversal_threads ? tuning.traversal_threads : 1024u;
+  ls.samples = ch.sample_count;
   const uint32_t cut_depth = std::max(1u, std::min(caps.trace_depth, 64u)) - 1u;
   ls.shade_sort = tuning.shade_sort == 2u   ? kShadeSortNone
                   : tuning.shade_sort == 3u ? kShadeSortBlock

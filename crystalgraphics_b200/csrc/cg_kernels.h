@@ -119,6 +119,7 @@ struct LaunchShape {
   bool persistent = true;    // persistent warps with lane refill
   bool spec = false;         // with persistent four-wide closest hits: postponed leaves
   uint32_t traversal_threads = 1024;  // threads per SM of the persistent traversal grids
+  uint32_t samples = 0xffffffffu;     // camera samples of the chunk (launchExtend's choice of walk)
   int shade_sort = kShadeSortGlobal;  // ShadeSort: order of the rays the shading kernel takes
 };
 

@@ -182,6 +182,7 @@ struct SceneView {
   uint32_t instance_count;
   uint32_t has_tlas;
   uint32_t has_lights;
+  uint32_t nodes4;             // four-wide nodes of all BLAS and the TLAS
 };
 
 }  // namespace cg

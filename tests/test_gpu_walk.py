@@ -66,3 +66,33 @@ def test_walk_matches_the_oracle(loaded):
     keep = ~primary_tie_mask(o, s.camera, w, h)
     close, rel_mean, _ = keyed_compare(out, ref, keep)
     assert close >= 0.995  # the criterion of the other keyed frames
+
+
+# ---- teams: the end of a small launch on deep trees ----------------------------------
+@pytest.fixture(scope="module", params=["mesh", "coincident"])
+def deep(request):
+    """A mesh of 327,680 triangles (launches of up to 2^20 samples let idle lanes
+    help), once with a second instance of another material in the same place,
+    so that two triangles are at every hit's distance."""
+    s = scenes.icosphere_scene(subdiv=7)
+    if request.param == "coincident":
+        twin = s.instances[:1].copy()
+        twin["material"] = 1
+        s.instances = np.ascontiguousarray(np.concatenate([s.instances, twin]))
+    B.EnvInit(B.PathTraceConf(render_width=8, render_height=8))
+    g = B.LoadScene(s)
+    yield s, g
+    g.close()
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (17, 2, 1), (33, 1, 3), (127, 3, 1), (320, 180, 2),
+                                  (1024, 1023, 1), (1024, 1024, 1), (1025, 1024, 1)])
+def test_teams_match_one_ray_per_thread(deep, size):
+    s, g = deep
+    w, h, spp = size
+    for k, camera in enumerate((B.Camera.from_c(s.camera),
+                                B.Camera((0.0, -1.35, 0.9), (0.0, 0.83, -0.55), (0.8, 0.45)))):
+        ref = frame(g, camera, w, h, spp, 8, persistent=False)
+        out = frame(g, camera, w, h, spp, 8, persistent=True)
+        scale = np.maximum(np.abs(ref), np.abs(ref).mean())
+        assert float((np.abs(out.astype(np.float64) - ref) / scale).max()) <= RTOL
