@@ -107,9 +107,12 @@ static int buildBatch(Env& env, const SceneDev& scene, const cg_view_desc* views
   return CG_OK;
 }
 
-// Renders a batch on env.stream; leaves the films on the device in `gp`.
+// Renders a batch on env.stream; leaves the films on the device in `gp`.  The
+// pages of the host buffer the films will be read into (may be null) are
+// populated while the device works.
 static int runBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, uint32_t n,
-                    BatchGraph*& gp, RenderRecord& rec, float& ms) {
+                    BatchGraph*& gp, RenderRecord& rec, float& ms, void* host = nullptr,
+                    size_t host_bytes = 0) {
   const Caps caps = capsOf(env.conf);
   int rc = env.ensureWave(env.tuning.queue_capacity);
   if (rc != CG_OK) return rc;
@@ -153,6 +156,7 @@ static int runBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, 
       rc = env.enqueueViews(scene, vd, table, caps, env.stream, fresh->rec);
       if (rc != CG_OK) return rc;
       CG_CUDA(cudaEventRecord(env.ev1, env.stream));
+      if (host) prefaultHostBuffer(host, host_bytes);
       CG_CUDA(cudaEventSynchronize(env.ev1));
       cudaEventElapsedTime(&ms, env.ev0, env.ev1);
       rec = fresh->rec;
@@ -168,6 +172,7 @@ static int runBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, 
   CG_CUDA(cudaEventRecord(env.ev0, env.stream));
   CG_CUDA(cudaGraphLaunch(gp->exec, env.stream));
   CG_CUDA(cudaEventRecord(env.ev1, env.stream));
+  if (host) prefaultHostBuffer(host, host_bytes);
   CG_CUDA(cudaEventSynchronize(env.ev1));
   cudaEventElapsedTime(&ms, env.ev0, env.ev1);
   rec = gp->rec;
@@ -195,34 +200,30 @@ CG_API int cg_batch_render(cg_scene_t scene, const cg_view_desc* views, uint32_t
     BatchGraph* g = nullptr;
     RenderRecord rec;
     float ms = 0.0f;
-    rc = runBatch(env, *s, views, view_count, g, rec, ms);
+    size_t npx = 0;
+    for (uint32_t i = 0; i < view_count; ++i) npx += size_t(views[i].width) * views[i].height;
+    rc = runBatch(env, *s, views, view_count, g, rec, ms, films_xyz, npx * 12);
     if (rc != CG_OK) return rc;
     rc = env.fetchStats(env.stream, rec);
     if (rc != CG_OK) return rc;
     CG_CUDA(cudaStreamSynchronize(env.stream));
     rc = env.readStats(rec, ms, env.last);
     if (rc != CG_OK) return rc;
-    // readback
+    // readback: the films packed on the device (in the shadow queue, idle now)
+    // and copied as one run, in slices where they exceed the queue
     const char* base = static_cast<const char*>(g->films.base);
     if (films_xyz) {
-      size_t total = 0;
-      for (uint32_t i = 0; i < view_count; ++i) total += size_t(views[i].width) * views[i].height;
-      std::vector<float> tmp;
-      size_t out = 0;
-      for (uint32_t i = 0; i < view_count; ++i) {
-        const size_t npx = size_t(views[i].width) * views[i].height;
-        tmp.resize(npx * 4);
-        CG_CUDA(cudaMemcpyAsync(tmp.data(), base + g->film_off[i], npx * 16, cudaMemcpyDeviceToHost,
+      const ViewDev* table = reinterpret_cast<const ViewDev*>(base + g->table_off);
+      float* packed = reinterpret_cast<float*>(env.wave.sh_o);
+      const size_t slice = env.wave.capacity;
+      for (size_t at = 0; at < npx; at += slice) {
+        const size_t count = std::min(slice, npx - at);
+        launchBatchPack(table, view_count, packed, at, count, env.stream);
+        CG_CUDA(cudaGetLastError());
+        CG_CUDA(cudaMemcpyAsync(films_xyz + 3 * at, packed, count * 12, cudaMemcpyDeviceToHost,
                                 env.stream));
-        CG_CUDA(cudaStreamSynchronize(env.stream));
-        for (size_t p = 0; p < npx; ++p) {
-          films_xyz[3 * (out + p)] = tmp[4 * p];
-          films_xyz[3 * (out + p) + 1] = tmp[4 * p + 1];
-          films_xyz[3 * (out + p) + 2] = tmp[4 * p + 2];
-        }
-        out += npx;
       }
-      (void)total;
+      CG_CUDA(cudaStreamSynchronize(env.stream));
     }
     if (films_rgba8) {
       size_t out = 0;

@@ -143,6 +143,10 @@ void launchResolve(const FrameConst& fc, const WaveBuffers& wb, const ChunkDesc&
                    cudaStream_t s);
 // Packs a float4 film to three floats per pixel (XYZ, or linear sRGB).
 void launchFilmPack(const float4* film, float* out, size_t npx, bool rgb, cudaStream_t s);
+// XYZ of pixels [begin, begin + npx) of a batch (its view table `views` as
+// layoutViews numbers them), three floats per pixel.
+void launchBatchPack(const ViewDev* views, uint32_t count, float* out, uint64_t begin, size_t npx,
+                     cudaStream_t s);
 // Re-resolves the rgba8 film from the float4 XYZ film (the resolve's sRGB step).
 void launchFilmRgba8(const float4* film, uchar4* rgba, size_t npx, cudaStream_t s);
 void launchTraceClosest(const SceneView& sc, const float4* rays, uint32_t n, float4* out_tuv,

@@ -75,3 +75,23 @@ def test_statistics_start_at_zero_in_every_run():
         assert B.LastStats().extend_rays == many[0]
     g.close()
     B.EnvTerm()
+
+
+@pytest.mark.parametrize("capacity", [4096, 4097, 1 << 20])
+def test_batch_films_read_in_slices(capacity):
+    """A batch's films come back packed through the shadow queue: in one run, in
+    several, and with a slice ending inside a view."""
+    s = scenes.cornell(32, 32)
+    B.EnvInit(B.PathTraceConf(render_width=8, render_height=8, trace_depth=3))
+    g = B.LoadScene(s)
+    sizes = [(64, 64), (1, 1), (91, 47), (33, 2), (64, 65)]
+    views = [((0.0, -3.4, 1.0), (0.0, 1.0, 0.0), w, h, 2, 5 + k) for k, (w, h) in enumerate(sizes)]
+    B.SetTuning(queue_capacity=capacity)
+    for _ in range(2):  # captured, replayed
+        films = B.batch_render(g, views)
+        for k, (w, h) in enumerate(sizes):
+            assert films[k].shape == (h, w, 3)
+            alone = B.batch_render(g, views[k:k + 1])[0]
+            assert close(films[k], alone) <= RTOL
+    g.close()
+    B.EnvTerm()
