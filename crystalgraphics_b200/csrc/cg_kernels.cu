@@ -1151,6 +1151,16 @@ template <int kSort, int kLobes, bool kHero, bool kLight = true, bool kDefer = f
 __device__ __forceinline__ void shadeLevel(const SceneView& sc, const FrameConst& fc,
                                            const WaveBuffers& wb, int depth, int parity) {
   stageSmitsTables();
+  // kStep: the block's warps take each slice together.  These kernels are bound
+  // by instruction fetch (92 to 244 KB of straight code a slice, 1.5-8 cycles
+  // without an instruction per issue): warps in step share what is fetched, and
+  // larger blocks more so (launchShade).  Shading, blocks of 128 without the
+  // barrier -> 512 with it: Cornell room, hero wavelengths 1.58 -> 1.32 ms a
+  // frame, textured room 0.80 -> 0.72; icosphere and instanced scene the same.
+  // With transmission lobes, where the lanes' paths differ more, it gains nothing
+  // (icosphere 6.99 -> 7.01, hero wavelengths 12.65 -> 12.99).
+  constexpr bool kStep =
+      kSort == kShadeSortGlobal && (kLobes & kLobeHit) && !(kLobes & kLobeTransmit);
   const uint32_t n = min(wb.counts[parity], wb.capacity);
   // [lo, hi): the queue slice (or, in global order, the permutation range of
   // this launch's keys) the launch takes
@@ -1175,6 +1185,7 @@ __device__ __forceinline__ void shadeLevel(const SceneView& sc, const FrameConst
     wb.counts[3] = 0u;
   for (uint32_t bbase = lo + blockIdx.x * blockDim.x; bbase < hi; bbase += gridDim.x * blockDim.x) {
     uint32_t i = bbase + threadIdx.x;
+    if constexpr (kStep) __syncthreads();
     if (kSort == kShadeSortGlobal) i = i < hi ? wb.shade_perm[i] : n;  // n: no ray
     if (kSort == kShadeSortBlock) {
       const int key = i < n ? shadeKeyOf(sc, wb.hit_inst[i], static_cast<uint32_t>(depth) >= cut_depth)
@@ -1809,24 +1820,30 @@ int launchShade(const SceneView& sc, const FrameConst& fc, const WaveBuffers& wb
                 int parity, const LaunchShape& ls, cudaStream_t s, bool light) {
   const uint32_t block = ls.shade_block > 256u ? 256u : ls.shade_block;
   const uint32_t grid = ls.grid_shade ? ls.grid_shade : gridFor(1024u / block);
+  // The opaque launches that step together (shadeLevel, kStep) take blocks four
+  // times as large, as far as the registers allow: 64 in the light-free kernels,
+  // at most 128 in the hero kernels.  The ones with the light sample (80
+  // registers) would lose a third of their warps: icosphere 6.97 -> 7.03 ms.
+  const uint32_t step_block = std::min(512u, 4u * block);
+  const uint32_t step_grid = ls.grid_shade ? ls.grid_shade : gridFor(1024u / step_block);
   constexpr int kOpaque = kLobeHit | kLobeDiffuse | kLobeReflect;
   const bool rr = fc.roulette != 0u && static_cast<uint32_t>(depth) >= fc.roulette;
   if (wb.hero) {  // hero-wavelength mode: level-wide order, one launch per lobe group
     k_shade_scatter<<<gridFor(4u), kScatterBlock, 0, s>>>(wb, parity);
     if (light && wb.defer && wb.defer_dist && wb.defer_w && !rr) {  // light-pdf terms in a pass
       k_shade_hero<0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      k_shade_hero<kOpaque, true, true><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
       k_shade_hero<kLobesAll, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
       k_light_pdf<<<gridFor(8u), 256, 0, s>>>(sc, wb, parity ^ 1);
       return 5;
     }
     if (light) {
       k_shade_hero<0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      k_shade_hero<kOpaque><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
       k_shade_hero<kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     } else {
       k_shade_hero<0, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      k_shade_hero<kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
       k_shade_hero<kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     }
     return 4;
@@ -1849,7 +1866,7 @@ int launchShade(const SceneView& sc, const FrameConst& fc, const WaveBuffers& wb
       k_shade<kShadeSortGlobal, kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     } else {
       k_shade<kShadeSortGlobal, 0, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kOpaque, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      k_shade<kShadeSortGlobal, kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
       k_shade<kShadeSortGlobal, kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     }
     return 4;
