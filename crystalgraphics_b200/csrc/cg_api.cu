@@ -176,6 +176,8 @@ int uploadScene(const HostScene& h, SceneDev& s) {
   v.emissive_count = static_cast<uint32_t>(h.eprim.size());
   v.instance_count = static_cast<uint32_t>(h.inst.size());
   v.nodes4 = static_cast<uint32_t>(h.blas4.size() + h.tlas4.size());
+  v.kinds = 0u;
+  for (const DevInstance& i : h.inst) v.kinds |= 1u << i.kind;
   v.has_tlas = h.inst.empty() ? 0u : 1u;
   v.has_lights = h.eprim.empty() ? 0u : 1u;
   s.eprim_off = parts[7].off;
@@ -488,7 +490,8 @@ void Renderer::enqueueChunk(const SceneDev& scene, uint32_t view_count, const Vi
     profEnd(s);
     profBegin(CG_K_SHADE, s);
     const int shade_kernels =
-        launchShade(scene.view, fc, wb, static_cast<int>(d), parity, ls, s, plan.shadow[d]);
+        launchShade(scene.view, fc, wb, static_cast<int>(d), parity, ls, s, plan.shadow[d],
+                    d >= cut_depth);
     profEnd(s);
     rec.launches += 1 + static_cast<uint32_t>(shade_kernels);
     if (plan.shadow[d]) {

@@ -163,7 +163,8 @@ __device__ __forceinline__ void beginShadeKeys() {
   __syncthreads();
 }
 
-// keys: 0 none, 1 keys for a level shaded before the depth cut, 2 after it.
+// keys: 0 none, 1 keys for a level shaded before the depth cut, 2 after it (any
+// hit is then key 1; the launches leave the keys of such a level out).
 // Called together by the lanes `lanes`, which finished a ray (one shared-memory
 // atomic per distinct key among them).
 __device__ __forceinline__ void writeShadeKey(const SceneView& sc, const WaveBuffers& wb, uint32_t i,
@@ -1564,13 +1565,13 @@ __global__ void __maxnreg__(kDefer ? CG_SHADE_DEFER_REGS : kLight ? 96 : CG_SHAD
   shadeLevel<kSort, kLobes, false, kLight, kDefer>(sc, fc, wb, depth, parity);
 }
 
-// Hero-wavelength mode (level-wide shading order only).  At most 128
+// Hero-wavelength mode (level-wide shading order, and the last level in none).  At most 128
 // registers: the group with transmission needs 109 without spills (ptxas
 // chose 96 with spills when left free).
-template <int kLobes, bool kLight = true, bool kDefer = false>
+template <int kLobes, bool kLight = true, bool kDefer = false, int kSort = kShadeSortGlobal>
 __global__ void __maxnreg__(128) k_shade_hero(SceneView sc, FrameConst fc, WaveBuffers wb,
                                                     int depth, int parity) {
-  shadeLevel<kShadeSortGlobal, kLobes, true, kLight, kDefer>(sc, fc, wb, depth, parity);
+  shadeLevel<kSort, kLobes, true, kLight, kDefer>(sc, fc, wb, depth, parity);
 }
 
 // Completes the weights of the children a light-sampling level deferred
@@ -1772,7 +1773,7 @@ bool teamShadow(const SceneView& sc) { return deepTrees(sc); }
 
 void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool counting,
                   const LaunchShape& ls, bool cut, cudaStream_t s) {
-  const int keys = ls.shade_sort == kShadeSortGlobal ? (cut ? 2 : 1) : 0;
+  const int keys = ls.shade_sort == kShadeSortGlobal && !cut ? 1 : 0;
   const uint32_t block = ls.extend_block;
   if (ls.persistent) {  // one resident grid: 64 registers -> 65536 / (64 * block) blocks per SM
     const uint32_t g = gridFor(std::max(1u, ls.traversal_threads / block));
@@ -1817,7 +1818,7 @@ void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool c
 }
 
 int launchShade(const SceneView& sc, const FrameConst& fc, const WaveBuffers& wb, int depth,
-                int parity, const LaunchShape& ls, cudaStream_t s, bool light) {
+                int parity, const LaunchShape& ls, cudaStream_t s, bool light, bool cut) {
   const uint32_t block = ls.shade_block > 256u ? 256u : ls.shade_block;
   const uint32_t grid = ls.grid_shade ? ls.grid_shade : gridFor(1024u / block);
   // The opaque launches that step together (shadeLevel, kStep) take blocks four
@@ -1828,48 +1829,70 @@ int launchShade(const SceneView& sc, const FrameConst& fc, const WaveBuffers& wb
   const uint32_t step_grid = ls.grid_shade ? ls.grid_shade : gridFor(1024u / step_block);
   constexpr int kOpaque = kLobeHit | kLobeDiffuse | kLobeReflect;
   const bool rr = fc.roulette != 0u && static_cast<uint32_t>(depth) >= fc.roulette;
+  // The last level needs no order: a hit there adds nothing, and misses are read
+  // best as queued.  One launch instead of a scatter and three groups.
+  if (cut && (wb.hero || ls.shade_sort == kShadeSortGlobal)) {
+    if (wb.hero)
+      k_shade_hero<0, false, false, kShadeSortNone><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+    else
+      k_shade<kShadeSortNone, 0, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+    return 1;
+  }
+  // Groups that no material of the scene falls into are not launched (an empty
+  // launch costs ~3 us; the 256x256 Cornell frame, without transmission, has
+  // two levels).
+  const bool opaque = (sc.kinds & 0x00ffu) != 0u, transmit = (sc.kinds & 0xff00u) != 0u;
+  const int groups = 1 + (opaque ? 1 : 0) + (transmit ? 1 : 0);
   if (wb.hero) {  // hero-wavelength mode: level-wide order, one launch per lobe group
     k_shade_scatter<<<gridFor(4u), kScatterBlock, 0, s>>>(wb, parity);
     if (light && wb.defer && wb.defer_dist && wb.defer_w && !rr) {  // light-pdf terms in a pass
       k_shade_hero<0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque, true, true><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kLobesAll, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque)
+        k_shade_hero<kOpaque, true, true><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit)
+        k_shade_hero<kLobesAll, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
       k_light_pdf<<<gridFor(8u), 256, 0, s>>>(sc, wb, parity ^ 1);
-      return 5;
+      return groups + 2;
     }
     if (light) {
       k_shade_hero<0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque) k_shade_hero<kOpaque><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit) k_shade_hero<kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     } else {
       k_shade_hero<0, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade_hero<kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque)
+        k_shade_hero<kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit) k_shade_hero<kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     }
-    return 4;
+    return groups + 1;
   }
   if (ls.shade_sort == kShadeSortGlobal) {  // keys and counts came with the closest hits
     k_shade_scatter<<<gridFor(4u), kScatterBlock, 0, s>>>(wb, parity);
-    // one launch per lobe group, each over its keys' range of the permutation
+    // one launch per lobe group, each over its keys' range of the permutation;
     // the light-pdf terms in a separate pass (not where roulette needs the
     // final weights)
     if (light && wb.defer && wb.defer_dist && !rr) {
       k_shade<kShadeSortGlobal, 0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kOpaque, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kLobesAll, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque)
+        k_shade<kShadeSortGlobal, kOpaque, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit)
+        k_shade<kShadeSortGlobal, kLobesAll, true, true><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
       k_light_pdf<<<gridFor(8u), 256, 0, s>>>(sc, wb, parity ^ 1);
-      return 5;
+      return groups + 2;
     }
     if (light) {
       k_shade<kShadeSortGlobal, 0><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kOpaque><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque) k_shade<kShadeSortGlobal, kOpaque><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit)
+        k_shade<kShadeSortGlobal, kLobesAll><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     } else {
       k_shade<kShadeSortGlobal, 0, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
-      k_shade<kShadeSortGlobal, kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (opaque)
+        k_shade<kShadeSortGlobal, kOpaque, false><<<step_grid, step_block, 0, s>>>(sc, fc, wb, depth, parity);
+      if (transmit)
+        k_shade<kShadeSortGlobal, kLobesAll, false><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);
     }
-    return 4;
+    return groups + 1;
   }
   if (ls.shade_sort == kShadeSortBlock)
     k_shade<kShadeSortBlock><<<grid, block, 0, s>>>(sc, fc, wb, depth, parity);

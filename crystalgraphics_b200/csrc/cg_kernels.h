@@ -127,16 +127,16 @@ void launchWavelengthTree(float* tree, float* consts, cudaStream_t s);
 void launchGen(const FrameConst& fc, const WaveBuffers& wb, const ChunkDesc& ch, cudaStream_t s);
 // With the level-wide shading order (ls.shade_sort == kShadeSortGlobal) the
 // launch also writes the level's shading keys; `cut`: the level is shaded at
-// or beyond the depth cut.
+// or beyond the depth cut, where only misses add anything and no order is needed.
 void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool counting,
                   const LaunchShape& ls, bool cut, cudaStream_t s);
-// Returns the number of kernels launched (one, or with the global sort the
-// scatter and one shading launch per lobe group: four, and k_light_pdf after
-// them on a light-sampling level with wb.defer set: five).
+// Returns the number of kernels launched: one, or with the global sort the
+// scatter, one shading launch per lobe group that the scene's materials can
+// need, and k_light_pdf after them on a light-sampling level with wb.defer set.
 // `light`: the level can draw light samples (false leaves the light-sample code
-// out of the level's global-order shading launches).
+// out of the level's global-order shading launches); `cut`: launchExtend's.
 int launchShade(const SceneView& sc, const FrameConst& fc, const WaveBuffers& wb, int depth,
-                int parity, const LaunchShape& ls, cudaStream_t s, bool light = true);
+                int parity, const LaunchShape& ls, cudaStream_t s, bool light, bool cut);
 void launchShadow(const SceneView& sc, const WaveBuffers& wb, bool counting,
                   const LaunchShape& ls, cudaStream_t s);
 void launchResolve(const FrameConst& fc, const WaveBuffers& wb, const ChunkDesc& ch,

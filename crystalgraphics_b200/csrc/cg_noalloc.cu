@@ -273,7 +273,7 @@ extern "C" CG_API int cg_render_noalloc(cg_scene_t scene, const cg_conf* conf,
       for (uint32_t d = 0; d < plan.levels; ++d) {
         const int parity = static_cast<int>(d & 1u);
         launchExtend(sd.view, wb, parity, false, ls, d >= cut_depth, s);
-        launchShade(sd.view, fc, wb, static_cast<int>(d), parity, ls, s);
+        launchShade(sd.view, fc, wb, static_cast<int>(d), parity, ls, s, true, d >= cut_depth);
         if (plan.shadow[d]) launchShadow(sd.view, wb, false, ls, s);
       }
       launchResolve(fc, wb, ch, s);

@@ -183,6 +183,7 @@ struct SceneView {
   uint32_t has_tlas;
   uint32_t has_lights;
   uint32_t nodes4;             // four-wide nodes of all BLAS and the TLAS
+  uint32_t kinds;              // shading kinds of the instances' materials (a bit each)
 };
 
 }  // namespace cg
