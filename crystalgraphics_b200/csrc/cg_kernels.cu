@@ -344,15 +344,16 @@ __device__ __forceinline__ void persistentTraverse(const SceneView& sc, WaveBuff
       fin = travStepsSpec<kCount, kNodes == kNodesWide4Q>(sc, st, leaf, stack, kStepBudget, cnt,
                                                           wb.status, ray >= 0);
     } else {
-      fin = ray >= 0 && travSteps<kAny, kCount, kNodes>(sc, st, stack, kStepBudget, cnt, wb.status);
+      fin = ray >= 0 && travSteps<kAny, kCount>(sc, st, stack, kStepBudget, cnt, wb.status);
     }
+    const unsigned fins = __ballot_sync(kFull, ray >= 0 && fin);
     if (ray >= 0 && fin) {
       if (kAny) {
         if (st.best.inst < 0) addShadowTerm(wb, static_cast<uint32_t>(ray));
       } else {
         wb.hit[ray] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
         wb.hit_inst[ray] = st.best.inst;
-        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, keys, __activemask());
+        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, keys, fins);
       }
       ray = -1;
     }

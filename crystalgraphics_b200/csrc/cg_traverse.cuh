@@ -359,57 +359,14 @@ struct ShortStack {
   }
 };
 
-// Runs at most `budget` steps (a node visit, a leaf, or a return to the
-// TLAS); returns true when the ray is finished (s.best holds its hit; with
+// Binary trees: runs at most `budget` steps (a node visit, a leaf, or a return
+// to the TLAS); returns true when the ray is finished (s.best holds its hit; with
 // kAny the first hit below s.best.t finishes it).
-template <bool kAny, bool kCount, int kNodes, class Stack>
+template <bool kAny, bool kCount, class Stack>
 __device__ __forceinline__ bool travSteps(const SceneView& sc, TravState& s, Stack& stack,
                                           int budget, TravCounters& cnt, uint32_t* status) {
   for (int step = 0; step < budget; ++step) {
     const int32_t node = s.node;
-    if (kNodes != kNodesBinary && node >= 0) {  // a four-wide node (traceRay4's inner step)
-      using W = Wide<kNodes == kNodesWide4Q>;
-      const typename W::Node* nodes = s.cur_inst < 0 ? W::tlas(sc) : W::blas(sc);
-      float nxs[4], fxs[4], nys[4], fys[4], nzs[4], fzs[4];
-      const int4 ch = W::fetch(nodes, node, s.idx < 0.0f, s.idy < 0.0f, s.idz < 0.0f, nxs, fxs,
-                               nys, fys, nzs, fzs);
-      if (kCount) ++cnt.nodes;
-      float k[4];
-      const int32_t links[4] = {ch.x, ch.y, ch.z, ch.w};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float a0 = fmaf(nxs[c], s.idx, -s.oix), a1 = fmaf(fxs[c], s.idx, -s.oix);
-        const float b0 = fmaf(nys[c], s.idy, -s.oiy), b1 = fmaf(fys[c], s.idy, -s.oiy);
-        const float c0 = fmaf(nzs[c], s.idz, -s.oiz), c1 = fmaf(fzs[c], s.idz, -s.oiz);
-        const float tmin = fmaxf(fmaxf(a0, b0), fmaxf(c0, 0.0f));
-        const float tmx = fminf(fminf(a1, b1), fminf(c1, s.best.t));
-        const bool hit = kNodes == kNodesWide4Q ? (tmin <= tmx && links[c] != kEmptyLink)
-                                                : tmin <= tmx;
-        k[c] = hit ? tmin : INFINITY;
-      }
-      int32_t l0 = ch.x, l1 = ch.y, l2 = ch.z, l3 = ch.w;
-      float k0 = k[0], k1 = k[1], k2 = k[2], k3 = k[3];
-      cswap(k0, l0, k1, l1);
-      cswap(k2, l2, k3, l3);
-      cswap(k0, l0, k2, l2);
-      cswap(k1, l1, k3, l3);
-      cswap(k1, l1, k2, l2);
-      if (k0 == INFINITY) {
-        s.node = s.sp > 0 ? stack.get(--s.sp) : kDone;
-        continue;
-      }
-      const int pushes = (k1 != INFINITY) + (k2 != INFINITY) + (k3 != INFINITY);
-      if (s.sp + pushes > kStackSize) {
-        atomicOr(status, 1u);
-        s.best = HitRec{s.best.t, 0.0f, 0.0f, -1, 0u};
-        return true;
-      }
-      if (k3 != INFINITY) stack.set(s.sp++, l3);
-      if (k2 != INFINITY) stack.set(s.sp++, l2);
-      if (k1 != INFINITY) stack.set(s.sp++, l1);
-      s.node = l0;
-      continue;
-    }
     if (node >= 0) {
       const BvhNode* nodes = s.cur_inst < 0 ? sc.tlas : sc.blas;
       const float4* np = reinterpret_cast<const float4*>(nodes + node);
@@ -480,8 +437,7 @@ __device__ __forceinline__ bool travSteps(const SceneView& sc, TravState& s, Sta
       }
       stack.set(s.sp++, kToTlas);
       s.cur_inst = static_cast<int32_t>(first);
-      // blas_root (binary) or blas4_root (four-wide)
-      s.node = static_cast<int32_t>(kNodes == kNodesBinary ? meta.x : meta.w);
+      s.node = static_cast<int32_t>(meta.x);  // blas_root
       continue;
     }
     for (uint32_t k = 0; k < count; ++k) {
@@ -503,7 +459,7 @@ __device__ __forceinline__ bool travSteps(const SceneView& sc, TravState& s, Sta
   return false;
 }
 
-// The closest-hit walk of travSteps over four-wide trees with postponed
+// The resumable closest-hit walk over four-wide trees with postponed
 // leaves ("speculative traversal", Aila & Laine 2009): a lane that reaches a
 // BLAS leaf parks it and goes on with its next inner node; the parked
 // triangles are tested when no lane of the warp still walks inner nodes

@@ -445,10 +445,12 @@ typedef struct cg_tuning {
   uint32_t extend_block;  /* threads per block of the traversal launches: a
                              multiple of 32 in [32, 256] (default 128; 0 = keep) */
   uint32_t shade_block;   /* the same for the shading launch (larger values
-                             run as 256) */
+                             run as 256; opaque groups whose warps step
+                             together take up to four times as many) */
   uint32_t use_graph;   /* 1 (default) = capture the launch sequence as a CUDA
                            graph and replay it: per batch in cg_batch_render,
-                           per scene in cg_view (not while profiling);
+                           per scene in cg_view (from a scene's second frame
+                           on, not while profiling);
                            always written (0 = launch directly) */
   uint32_t bvh_width;   /* 4 (default) or 2: node width the traversal walks */
   uint32_t persistent;  /* 1 (default) = persistent traversal warps that refill
