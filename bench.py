@@ -66,9 +66,9 @@ FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 # launch's traffic is taken as proportional to its rays (the trees stay
 # L2-resident at both sizes).  None where no capture of the variant exists.
 EXTEND_COUNTERS = {
-    "dram_bytes_per_ray": 145.0,   # 2162 MB over the 14 launches of a frame of 14,915,514 rays
-    "l2_bytes_per_ray": 962.3,     # L2 / DRAM bytes 6.64 on two of those launches
-    "lanes_active": 10.4,          # 11.58 and 9.17 of 32 on the same two
+    "dram_bytes_per_ray": 145.9,   # 2176 MB over the 14 launches of a frame of 14,915,519 rays
+    "l2_bytes_per_ray": 1145.0,    # L2 / DRAM bytes 7.85 on two of those launches
+    "lanes_active": 17.9,          # 18.44 and 17.41 of 32 on the same two
 }
 
 
