@@ -490,6 +490,10 @@ __device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers
 
   while (true) {
     if (kTeam && exhausted) {  // what the team has found by now
+      // The bounds were lowered by other lanes' atomics in an earlier turn, and a
+      // ballot orders no memory: this orders them before the reads here and at
+      // the end of a walk below.
+      __syncwarp();
       const float b = __int_as_float(team(kTeamBound, team(kTeamHome, me)));
       if (kAny) {
         if (b == -INFINITY && ray >= 0 && node != kWait) {
