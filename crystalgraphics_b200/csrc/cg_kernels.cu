@@ -440,7 +440,7 @@ constexpr size_t walkBytes() {
 template <bool kAny, bool kCount, int kNodes, bool kTeam>
 __device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers& wb, uint32_t n,
                                           uint32_t* work, int parity, int keys) {
-  static_assert(kNodes != kNodesBinary);
+  static_assert(kNodes != kNodesBinary && !(kTeam && kCount));
   using W = Wide<kNodes == kNodesWide4Q>;
   const uint32_t lane = threadIdx.x & 31u;
   const int me = static_cast<int>(lane);
@@ -1768,6 +1768,8 @@ namespace {
 // longest: below 2^16 four-wide nodes helping costs more than it saves (one
 // icosphere, 921,600 samples, closest hit plain -> team: 22,000 nodes 1.31 ->
 // 1.40 ms, 88,000 nodes 1.56 -> 1.55, 352,000 nodes 2.19 -> 1.80).
+// Never with counting on: the counters are the one-ray walk's, and helpers visit
+// more, by an amount that depends on which lanes were free.
 bool deepTrees(const SceneView& sc) { return sc.nodes4 >= (1u << 16); }
 
 // Closest hits: the walk with teams is 2-4 % slower while the queue lasts, so
@@ -1806,10 +1808,9 @@ void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool c
       }
       return;
     }
-    if (ls.nodes == kNodesWide4 && teamExtend(sc, ls)) {
+    if (ls.nodes == kNodesWide4 && !counting && teamExtend(sc, ls)) {
       const size_t team = walkBytes<false, true>() * block;
-      if (counting) k_extend_persistent<true, kNodesWide4, false, true><<<g, block, team, s>>>(sc, wb, parity, keys);
-      else k_extend_persistent<false, kNodesWide4, false, true><<<g, block, team, s>>>(sc, wb, parity, keys);
+      k_extend_persistent<false, kNodesWide4, false, true><<<g, block, team, s>>>(sc, wb, parity, keys);
       return;
     }
     switch (ls.nodes * 2 + (counting ? 1 : 0)) {
@@ -1923,10 +1924,9 @@ void launchShadow(const SceneView& sc, const WaveBuffers& wb, bool counting,
   if (ls.persistent) {
     const uint32_t g = gridFor(std::max(1u, ls.traversal_threads / block));
     const size_t walk = walkBytes<true>() * block;
-    if (ls.nodes == kNodesWide4 && teamShadow(sc)) {
+    if (ls.nodes == kNodesWide4 && !counting && teamShadow(sc)) {
       const size_t team = walkBytes<true, true>() * block;
-      if (counting) k_shadow_persistent<true, kNodesWide4, true><<<g, block, team, s>>>(sc, wb);
-      else k_shadow_persistent<false, kNodesWide4, true><<<g, block, team, s>>>(sc, wb);
+      k_shadow_persistent<false, kNodesWide4, true><<<g, block, team, s>>>(sc, wb);
       return;
     }
     switch (ls.nodes * 2 + (counting ? 1 : 0)) {
