@@ -743,6 +743,7 @@ static int renderEnvView(Env& env, SceneDev* s, std::vector<ViewDev>& views, boo
         return rc;
       }
       if (ce != cudaSuccess) return cudaFail(ce, "cudaStreamEndCapture");
+      vg = env.makeRoom(r.launches);
       ce = cudaGraphInstantiate(&vg->exec, graph, 0);
       cudaGraphDestroy(graph);
       if (ce != cudaSuccess) {

@@ -228,8 +228,14 @@ struct Env : Renderer {
   // the statistics.  The first frame of a scene is launched directly (capturing
   // and instantiating takes longer than the launches save there), the second
   // one captures, later ones replay.  The kMaxViewGraphs scenes viewed last
-  // keep theirs; a tuning change drops all, a destroyed scene its own.
+  // keep theirs, as far as their launches come to kMaxViewGraphLaunches in all
+  // (the scene in view keeps its own at any size); a tuning change drops all, a
+  // destroyed scene its own.  A graph takes about 2.6 KB of device and 6.8 KB of
+  // host memory a launch (59,280 launches, a 1920x1080 frame in 1520 chunks: 150
+  // and 400 MB), so the limit keeps all of them within 60 and 160 MB or to one.
+  // A frame of one chunk has 20 to 60 launches.
   static constexpr size_t kMaxViewGraphs = 8;
+  static constexpr uint32_t kMaxViewGraphLaunches = 24576;
   struct ViewGraph {
     uint64_t scene_tag = 0;
     bool counting = false;
@@ -240,6 +246,9 @@ struct Env : Renderer {
   // The entry of a scene in the current counting mode, moved to the back; null
   // where there was none (an entry without a graph is added then)
   ViewGraph* viewGraphOf(uint64_t scene_tag);
+  // Drops the least recently viewed graphs until the others and one of
+  // `launches` launches, the back entry's, are within the limit.
+  ViewGraph* makeRoom(uint32_t launches);
   void dropViewGraphs();
 
   void dropGraphsFor(uint64_t tag);

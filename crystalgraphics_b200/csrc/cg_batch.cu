@@ -59,6 +59,20 @@ Env::ViewGraph* Env::viewGraphOf(uint64_t scene_tag) {
   view_graphs.push_back(g);
   return nullptr;
 }
+Env::ViewGraph* Env::makeRoom(uint32_t launches) {
+  uint64_t total = launches;
+  for (const ViewGraph& g : view_graphs)
+    if (g.exec) total += g.rec.launches;
+  while (view_graphs.size() > 1 && total > kMaxViewGraphLaunches) {
+    const ViewGraph& g = view_graphs.front();
+    if (g.exec) {
+      total -= g.rec.launches;
+      cudaGraphExecDestroy(g.exec);
+    }
+    view_graphs.erase(view_graphs.begin());
+  }
+  return &view_graphs.back();
+}
 
 // Builds the view table of a batch into `g` (films allocated per view).
 static int buildBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, uint32_t n,
