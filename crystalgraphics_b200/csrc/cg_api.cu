@@ -39,6 +39,12 @@ void prefaultHostBuffer(void* p, size_t bytes) {
 #endif
 }
 
+void prefaultUnlessPinned(void* p, size_t bytes) {
+  cudaPointerAttributes attr{};
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) cudaGetLastError();
+  if (attr.type != cudaMemoryTypeHost) prefaultHostBuffer(p, bytes);
+}
+
 thread_local std::string tl_error;
 
 int fail(int code, const std::string& msg) {
@@ -1091,11 +1097,7 @@ CG_API int cg_film_read(void* host, size_t bytes, int format) {
     Env& env = *g_env;
     const size_t npx = size_t(env.conf.render_width) * env.conf.render_height;
     CG_CUDA(cudaSetDevice(env.device));
-    // (a pinned buffer is mapped already)
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) cudaGetLastError();
-    if (attr.type != cudaMemoryTypeHost)
-      prefaultHostBuffer(host, std::min(bytes, npx * (format == CG_FILM_RGBA8 ? 4 : 12)));
+    prefaultUnlessPinned(host, std::min(bytes, npx * (format == CG_FILM_RGBA8 ? 4 : 12)));
     if (format == CG_FILM_RGBA8) {
       if (bytes < npx * 4) return fail(CG_E_INVALID, "buffer too small for RGBA8");
       CG_CUDA(cudaMemcpyAsync(host, env.rgba, npx * 4, cudaMemcpyDeviceToHost, env.stream));

@@ -170,7 +170,7 @@ static int runBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, 
       rc = env.enqueueViews(scene, vd, table, caps, env.stream, fresh->rec);
       if (rc != CG_OK) return rc;
       CG_CUDA(cudaEventRecord(env.ev1, env.stream));
-      if (host) prefaultHostBuffer(host, host_bytes);
+      if (host) prefaultUnlessPinned(host, host_bytes);
       CG_CUDA(cudaEventSynchronize(env.ev1));
       cudaEventElapsedTime(&ms, env.ev0, env.ev1);
       rec = fresh->rec;
@@ -186,7 +186,7 @@ static int runBatch(Env& env, const SceneDev& scene, const cg_view_desc* views, 
   CG_CUDA(cudaEventRecord(env.ev0, env.stream));
   CG_CUDA(cudaGraphLaunch(gp->exec, env.stream));
   CG_CUDA(cudaEventRecord(env.ev1, env.stream));
-  if (host) prefaultHostBuffer(host, host_bytes);
+  if (host) prefaultUnlessPinned(host, host_bytes);
   CG_CUDA(cudaEventSynchronize(env.ev1));
   cudaEventElapsedTime(&ms, env.ev0, env.ev1);
   rec = gp->rec;
