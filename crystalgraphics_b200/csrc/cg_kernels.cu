@@ -134,8 +134,8 @@ __global__ void k_gen(FrameConst fc, WaveBuffers wb, ChunkDesc ch) {
 }
 
 // ---- shading keys (the level-wide shading order) ---------------------------------
-// Key of a hit: 0 miss, 1 hit beyond the depth cut (no work), 2 + material
-// kind; kNumKeys - 1 marks an empty slot.  The closest-hit kernel writes each
+// Key of a hit: 0 miss, 1 hit beyond the depth cut (no work; only the per-block
+// order sorts such a level), 2 + material kind; kNumKeys - 1 marks an empty slot.  The closest-hit kernel writes each
 // ray's key and counts rays per key (counts[kKeyCount + k]); the block that
 // finishes last turns the counts into the scatter cursors (counts[kKeyCursor
 // + k], exclusive prefix sums) and zeroes the counts and the ticket
@@ -163,13 +163,11 @@ __device__ __forceinline__ void beginShadeKeys() {
   __syncthreads();
 }
 
-// keys: 0 none, 1 keys for a level shaded before the depth cut, 2 after it (any
-// hit is then key 1; the launches leave the keys of such a level out).
 // Called together by the lanes `lanes`, which finished a ray (one shared-memory
 // atomic per distinct key among them).
 __device__ __forceinline__ void writeShadeKey(const SceneView& sc, const WaveBuffers& wb, uint32_t i,
-                                              int32_t inst, int keys, unsigned lanes) {
-  const int key = shadeKeyOf(sc, inst, keys == 2);
+                                              int32_t inst, unsigned lanes) {
+  const int key = shadeKeyOf(sc, inst, false);
   wb.shade_key[i] = static_cast<uint8_t>(key);
   const unsigned peers = __match_any_sync(lanes, key);
   if ((threadIdx.x & 31u) == static_cast<uint32_t>(__ffs(peers) - 1))
@@ -226,7 +224,7 @@ __device__ __forceinline__ HitRec trace(const SceneView& sc, float4 o, float4 d,
 // keys (writeShadeKey): also the level's shading keys and their counts.
 template <bool kCount, int kNodes>
 __global__ void __launch_bounds__(256, 4) k_extend(SceneView sc, WaveBuffers wb, int parity,
-                                                   int keys) {
+                                                   bool keys) {
   // counts can exceed the capacity after an overflow (the appends are then
   // dropped and the status word set); never read past the queue
   const uint32_t n = min(wb.counts[parity], wb.capacity);
@@ -246,7 +244,7 @@ __global__ void __launch_bounds__(256, 4) k_extend(SceneView sc, WaveBuffers wb,
     HitRec h = trace<false, kCount, kNodes>(sc, o, d, MAXD, cnt, wb.status);
     wb.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.tri));
     wb.hit_inst[i] = h.inst;
-    if (keys) writeShadeKey(sc, wb, i, h.inst, keys, __activemask());
+    if (keys) writeShadeKey(sc, wb, i, h.inst, __activemask());
   }
   if (keys) finishShadeKeys(wb);
   if (kCount) {
@@ -302,7 +300,7 @@ constexpr int kShortStack = 16;
 // kSpec: closest hits over four-wide trees with postponed leaves (travStepsSpec).
 template <bool kAny, bool kCount, int kNodes, bool kSpec = false>
 __device__ __forceinline__ void persistentTraverse(const SceneView& sc, WaveBuffers& wb, uint32_t n,
-                                                   uint32_t* work, int parity, int keys) {
+                                                   uint32_t* work, int parity, bool keys) {
   const uint32_t lane = threadIdx.x & 31u;
   TravCounters cnt{0u, 0u, 0u};
   extern __shared__ int32_t s_stack[];
@@ -353,7 +351,7 @@ __device__ __forceinline__ void persistentTraverse(const SceneView& sc, WaveBuff
       } else {
         wb.hit[ray] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
         wb.hit_inst[ray] = st.best.inst;
-        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, keys, fins);
+        if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), st.best.inst, fins);
       }
       ray = -1;
     }
@@ -439,7 +437,7 @@ constexpr size_t walkBytes() {
 // kAny: shadow rays (the first hit below a ray's bound ends it).
 template <bool kAny, bool kCount, int kNodes, bool kTeam>
 __device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers& wb, uint32_t n,
-                                          uint32_t* work, int parity, int keys) {
+                                          uint32_t* work, int parity, bool keys) {
   static_assert(kNodes != kNodesBinary && !(kTeam && kCount));
   using W = Wide<kNodes == kNodesWide4Q>;
   const uint32_t lane = threadIdx.x & 31u;
@@ -647,7 +645,7 @@ __device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers
           const int32_t inst = __float_as_int(s_hit[3 * bd]);
           wb.hit[ray] = make_float4(best, s_hit[0], s_hit[bd], s_hit[2 * bd]);
           wb.hit_inst[ray] = inst;
-          if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), inst, keys, fins);
+          if (keys) writeShadeKey(sc, wb, static_cast<uint32_t>(ray), inst, fins);
         }
         ray = -1;
       }
@@ -825,7 +823,7 @@ __device__ __forceinline__ void walkQueue(const SceneView& sc, const WaveBuffers
 #endif
 template <bool kCount, int kNodes, bool kSpec = false, bool kTeam = false>
 __global__ void CG_EXTEND_BOUNDS k_extend_persistent(SceneView sc, WaveBuffers wb,
-                                                              int parity, int keys) {
+                                                              int parity, bool keys) {
   const uint32_t n = min(wb.counts[parity], wb.capacity);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     wb.counts[parity ^ 1] = 0u;
@@ -846,9 +844,9 @@ __global__ void __launch_bounds__(256, 4) k_shadow_persistent(SceneView sc, Wave
   const uint32_t n = min(wb.counts[2], wb.capacity);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wb.stats[1], static_cast<unsigned long long>(n));
   if constexpr (kNodes == kNodesBinary)
-    persistentTraverse<true, kCount, kNodes>(sc, wb, n, &wb.counts[4], 0, 0);
+    persistentTraverse<true, kCount, kNodes>(sc, wb, n, &wb.counts[4], 0, false);
   else
-    walkQueue<true, kCount, kNodes, kTeam>(sc, wb, n, &wb.counts[4], 0, 0);
+    walkQueue<true, kCount, kNodes, kTeam>(sc, wb, n, &wb.counts[4], 0, false);
 }
 
 // ---- shadow: t-bounded any hit (solveEmission, trace.wesl:91-113) ----------------
@@ -1133,7 +1131,7 @@ __global__ void __launch_bounds__(kScatterBlock) k_shade_scatter(WaveBuffers wb,
 
 // kLobes: the lobe group (kLobesAll unless the level is in global shading
 // order, where one launch per group takes its keys' contiguous range of the
-// permutation: keys [0, 2) misses and hits beyond the depth cut, [2, 10) opaque
+// permutation: keys [0, 2) misses, [2, 10) opaque
 // kinds, [10, 18) kinds with transmission; see shadeKeyOf).
 // kSort (ShadeSort): kShadeSortBlock — before shading, every block sorts its
 // slice of the queue by shading key in shared memory (counting sort);
@@ -1791,7 +1789,7 @@ bool teamShadow(const SceneView& sc) { return deepTrees(sc); }
 
 void launchExtend(const SceneView& sc, const WaveBuffers& wb, int parity, bool counting,
                   const LaunchShape& ls, bool cut, cudaStream_t s) {
-  const int keys = ls.shade_sort == kShadeSortGlobal && !cut ? 1 : 0;
+  const bool keys = ls.shade_sort == kShadeSortGlobal && !cut;
   const uint32_t block = ls.extend_block;
   if (ls.persistent) {  // one resident grid: 64 registers -> 65536 / (64 * block) blocks per SM
     const uint32_t g = gridFor(std::max(1u, ls.traversal_threads / block));
