@@ -289,12 +289,13 @@ __device__ __forceinline__ void addShadowTerm(const WaveBuffers& wb, uint32_t i)
 #endif
 constexpr int kStepBudget = CG_STEP_BUDGET;
 constexpr int kRefill = CG_REFILL;
-// Closest-hit traversal stack entries per thread kept in shared memory
-// (dynamic shared memory of the persistent closest-hit launch: kShortStack * 4
-// bytes per thread).  Measured on the 1280x720 icosphere frame and the
-// instanced scene: closest-hit launches 1-2% faster than with the whole stack
-// in local memory, shadow launches 6-8% slower (their walks are short and the
-// shared carve-out costs them L1), so shadow rays keep a local stack.
+// Closest-hit stack entries per thread that this walk (binary trees and
+// postponed leaves; walkQueue has its own) keeps in shared memory (dynamic shared
+// memory of the launch: kShortStack * 4 bytes per thread).  Measured when it took
+// all launches, on the 1280x720 icosphere frame and the instanced scene:
+// closest-hit launches 1-2% faster than with the whole stack in local memory,
+// shadow launches 6-8% slower (their walks are short and the shared carve-out
+// costs them L1), so its shadow rays keep a local stack.
 constexpr int kShortStack = 16;
 
 // kSpec: closest hits over four-wide trees with postponed leaves (travStepsSpec).
@@ -1703,8 +1704,7 @@ __global__ void k_permute_rows(Node* nodes, size_t count) {
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= count) return;
   constexpr int kRows = sizeof(Node) / sizeof(uint4);
-  const uint32_t n = static_cast<uint32_t>(i);
-  const uint32_t place = kRows == 8 ? (n & 3u) << 1 : (n >> 1) & 3u;  // the walks' fetch
+  const uint32_t place = Wide<std::is_same_v<Node, Bvh4QNode>>::place(static_cast<uint32_t>(i));
   uint4* rows = reinterpret_cast<uint4*>(nodes + i);
   uint4 in[kRows];
 #pragma unroll
@@ -1765,7 +1765,14 @@ namespace {
 // Walks of deep trees differ most in length, and a launch ends with its
 // longest: below 2^16 four-wide nodes helping costs more than it saves (one
 // icosphere, 921,600 samples, closest hit plain -> team: 22,000 nodes 1.31 ->
-// 1.40 ms, 88,000 nodes 1.56 -> 1.55, 352,000 nodes 2.19 -> 1.80).
+// 1.40 ms, 88,000 nodes 1.56 -> 1.55, 352,000 nodes 1.99 -> 1.55).  The rule
+// counts the nodes of all trees, so it also takes scenes of many small meshes,
+// where it gains with the depth of the TLAS; closest hits plus shadow rays at
+// 57,600 / 230,400 / 921,600 samples, ms: 120,000 meshes of 20 triangles 1.72 ->
+// 1.59 / 2.49 -> 2.30 / 6.12 -> 6.12; 30,000 such 1.26 -> 1.20 / 1.73 -> 1.59 /
+// 3.59 -> 3.54; 12,000 of 80 triangles 0.94 -> 0.99 / 1.15 -> 1.17 / 1.86 -> 1.89;
+// 4,000 of 320 triangles, where it costs most, 0.58 -> 0.68 / 0.75 -> 0.83 / 0.94
+// -> 1.03.
 // Never with counting on: the counters are the one-ray walk's, and helpers visit
 // more, by an amount that depends on which lanes were free.
 bool deepTrees(const SceneView& sc) { return sc.nodes4 >= (1u << 16); }
@@ -1773,16 +1780,16 @@ bool deepTrees(const SceneView& sc) { return sc.nodes4 >= (1u << 16); }
 // Closest hits: the walk with teams is 2-4 % slower while the queue lasts, so
 // it takes launches whose end weighs more than that: chunks of up to 2^20
 // samples (icosphere / instanced scene, closest hit plain -> team, ms: 57,600
-// samples 1.10 -> 0.78 / 1.95 -> 1.97; 230,400 1.39 -> 1.05 / 2.63 -> 2.54;
-// 921,600 2.19 -> 1.80 / 5.73 -> 5.75; 1.8M 3.11 -> 2.87 / 9.83 -> 10.06; 7.4M
-// 8.83 -> 9.09 / 38.1 -> 39.1).
+// samples 1.06 -> 0.76 / 1.90 -> 1.93; 230,400 1.32 -> 0.92 / 2.55 -> 2.53;
+// 921,600 1.99 -> 1.55 / 4.79 -> 4.80; with the limit lifted 1.8M 3.11 -> 2.87 /
+// 9.83 -> 10.06; 7.4M 8.83 -> 9.09 / 38.1 -> 39.1).
 bool teamExtend(const SceneView& sc, const LaunchShape& ls) {
   return deepTrees(sc) && ls.samples <= (1u << 20);
 }
 
-// Shadow rays: at any size (57,600 samples 0.23 -> 0.17, 921,600 0.37 -> 0.28,
-// 7.4M 1.33 -> 1.31 on the icosphere; 0.17 -> 0.18, 0.27 -> 0.25 and 1.32 ->
-// 1.26 on the instanced scene).
+// Shadow rays: at any size (57,600 samples 0.27 -> 0.17, 921,600 0.37 -> 0.27,
+// 3.7M 0.76 -> 0.68 on the icosphere; 0.18 -> 0.17, 0.26 -> 0.25 and 0.62 ->
+// 0.57 on the instanced scene).
 bool teamShadow(const SceneView& sc) { return deepTrees(sc); }
 
 }  // namespace

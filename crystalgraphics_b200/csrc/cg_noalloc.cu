@@ -259,7 +259,7 @@ extern "C" CG_API int cg_render_noalloc(cg_scene_t scene, const cg_conf* conf,
     fc.caps = caps;
     fc.wl_tree = reinterpret_cast<const float*>(base + kOffWlTree);
     fc.wl_const = reinterpret_cast<const float*>(base + kOffWlConst);
-    LaunchShape ls;  // default block sizes
+    LaunchShape ls;  // default block sizes, and the closest-hit walk without helpers at any size
     const uint32_t cut_depth = std::max(1u, std::min(caps.trace_depth, 64u)) - 1u;
     uint64_t pix = 0, smp = 0;
     while (pix < npx) {  // the chunk sequence of Renderer::enqueueChunk

@@ -224,6 +224,7 @@ __device__ __forceinline__ void ldg256(const void* p, uint32_t w[8]) {
         "=r"(w[7])
       : "l"(p));
 }
+
 // The two four-wide node formats: full-precision child slabs, or 8-bit
 // offsets from the node origin (decoded to world-space bounds that contain
 // the full-precision ones: fmaf rounds q * scale + origin to nearest, and the
@@ -233,20 +234,23 @@ __device__ __forceinline__ void ldg256(const void* p, uint32_t w[8]) {
 // >= 0): the slab distances then need no min/max per axis.  With FMA rounding
 // monotonic in the bound, near <= far along the ray, so the entry and exit
 // distances equal min/max of the two slab planes bit for bit.
+// place(n): 16-byte row r of node n is at r ^ place(n) on the device
+// (launchPermuteNodes writes them there).
 template <bool kQuant>
 struct Wide;
 
 template <>
 struct Wide<false> {
   using Node = Bvh4Node;
+  // pairs of rows change places: p (lo and hi of an axis, or the links) to p ^ (n & 3)
+  static __device__ __forceinline__ uint32_t place(uint32_t n) { return (n & 3u) << 1; }
   static __device__ __forceinline__ const Node* tlas(const SceneView& sc) { return sc.tlas4; }
   static __device__ __forceinline__ const Node* blas(const SceneView& sc) { return sc.blas4; }
   static __device__ __forceinline__ int4 fetch(const Node* nodes, int32_t n, bool negx, bool negy,
                                                bool negz, float nx[4], float fx[4], float ny[4],
                                                float fy[4], float nz[4], float fz[4]) {
     const char* np = reinterpret_cast<const char*>(nodes + n);
-    // row pair p (lo and hi of an axis, or the links) is at place p ^ (n & 3)
-    const uint32_t sw = (static_cast<uint32_t>(n) & 3u) << 5;
+    const uint32_t sw = place(static_cast<uint32_t>(n)) * 16u;
     uint32_t x[8], y[8], z[8];
     ldg256(np + sw, x);
     ldg256(np + (sw ^ 32u), y);
@@ -268,13 +272,14 @@ struct Wide<false> {
 template <>
 struct Wide<true> {
   using Node = Bvh4QNode;
+  static __device__ __forceinline__ uint32_t place(uint32_t n) { return (n >> 1) & 3u; }
   static __device__ __forceinline__ const Node* tlas(const SceneView& sc) { return sc.tlas4q; }
   static __device__ __forceinline__ const Node* blas(const SceneView& sc) { return sc.blas4q; }
   static __device__ __forceinline__ int4 fetch(const Node* nodes, int32_t n, bool negx, bool negy,
                                                bool negz, float nx[4], float fx[4], float ny[4],
                                                float fy[4], float nz[4], float fz[4]) {
     const float4* np = reinterpret_cast<const float4*>(nodes + n);
-    const uint32_t sw = (static_cast<uint32_t>(n) >> 1) & 3u;  // row r at slot r ^ sw
+    const uint32_t sw = place(static_cast<uint32_t>(n));
     const float4 h = __ldg(np + sw);
     const uint4 qa = __ldg(reinterpret_cast<const uint4*>(np + (sw ^ 1u)));  // lo.x hi.x lo.y hi.y
     const uint4 qb = __ldg(reinterpret_cast<const uint4*>(np + (sw ^ 2u)));  // lo.z hi.z
@@ -603,7 +608,7 @@ __device__ __forceinline__ bool travStepsSpec(const SceneView& sc, TravState& s,
 }
 
 // The same closest / any hit over Bvh4Node trees: one node visit tests four
-// boxes (six independent 128-bit slab loads), the hit children are ordered
+// boxes (three independent 256-bit slab loads), the hit children are ordered
 // by entry distance, the nearest is visited next and the others pushed.
 // Triangle and instance handling is that of traceRay (bit-identical hits).
 template <bool kAny, bool kCount, bool kQuant = false>

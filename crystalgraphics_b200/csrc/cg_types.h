@@ -45,8 +45,8 @@ enum NodeFormat : int {
   kNodesWide4Q = 2,  // Bvh4QNode, four children with 8-bit boxes
 };
 
-// Four-wide node: the slabs of four children, structure-of-arrays so each
-// axis bound is one 128-bit load; links as in BvhNode (leaf count in the low
+// Four-wide node: the slabs of four children, structure-of-arrays so the two
+// bounds of an axis are one 256-bit load; links as in BvhNode (leaf count in the low
 // 3 bits of ~link).  An absent child has link kEmptyLink and a point box at
 // 1e30.  Collapsed from the SAH BVH2, it halves the dependent node fetches of
 // a ray.  On the device the four row pairs (lo and hi of one axis, and the
@@ -69,8 +69,9 @@ static_assert(sizeof(Bvh4Node) == 128, "Bvh4Node is 128 bytes");
 // (child lo = origin + qlo * scale <= the child's box, hi likewise >=), so a
 // quantised box always contains the full-precision one.  Same indices and
 // links as the Bvh4Node array it is built from; an absent child
-// (kEmptyLink) is skipped by its link, not by its box.  On the device row r of
-// node i is at place r ^ ((i >> 1) & 3), as for Bvh4Node.
+// (kEmptyLink) is skipped by its link, not by its box.  On the device its four
+// 16-byte rows are permuted for the same reason as Bvh4Node's row pairs, row r
+// of node i at place r ^ ((i >> 1) & 3).
 struct alignas(16) Bvh4QNode {
   float ox, oy, oz;
   uint32_t scale_bits;    // biased float exponents of the x, y, z scales (bytes 0..2)
