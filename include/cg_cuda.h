@@ -337,6 +337,8 @@ typedef struct cg_stats {
   uint64_t samples;          /* camera-path samples (pixels x spp)            */
   uint64_t extend_rays;      /* closest-hit rays traced (all depths)          */
   uint64_t shadow_rays;      /* shadow rays traced                            */
+  /* (counters of the traversal, those of the one-ray walk: the same in every
+   * run of the same samples) */
   uint64_t node_visits;      /* BVH node visits (counting build only, else 0) */
   uint64_t tri_tests;        /* triangle tests (counting build only, else 0)  */
   uint64_t inst_visits;      /* instance entries (counting build only, else 0)*/
