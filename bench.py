@@ -56,6 +56,8 @@ NODE_B = {4: 128, "4q": 64, 2: 64}
 TRI_B, INST_B, RAY_B = 48, 64, 52
 # non-tensor FP32 peak (nominal; no measured figure exists for it)
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
+# L1's data pipe, nominal: 128 bytes a cycle and SM
+L1_PEAK_GBS = 148 * 128 * 1.965e9 / 1e9
 # Memory traffic of the closest-hit kernel (k_extend_persistent, four-wide
 # float-box trees) per extend ray, from ncu on the medium icosphere case
 # (640x360, 16 spp, 16M-ray queues): DRAM bytes (dram__bytes_read.sum +
@@ -66,9 +68,9 @@ FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 # launch's traffic is taken as proportional to its rays (the trees stay
 # L2-resident at both sizes).  None where no capture of the variant exists.
 EXTEND_COUNTERS = {
-    "dram_bytes_per_ray": 145.9,   # 2176 MB over the 14 launches of a frame of 14,915,519 rays
-    "l2_bytes_per_ray": 1145.0,    # L2 / DRAM bytes 7.85 on two of those launches
-    "lanes_active": 17.9,          # 18.44 and 17.41 of 32 on the same two
+    "dram_bytes_per_ray": 146.2,   # 2180 MB over the 14 launches of a frame of 14,915,519 rays
+    "l2_bytes_per_ray": 1133.0,    # L2 / DRAM bytes 7.75 on two of those launches
+    "lanes_active": 18.0,          # 18.47 and 17.44 of 32 on the same two
 }
 
 
@@ -777,7 +779,7 @@ def run_ours(args):
         traffic = EXTEND_COUNTERS["dram_bytes_per_ray"] * rays_per_launch
         gbs = traffic / avg_launch_s / 1e9
         dram_side = {"bytes_per_launch": traffic, "achieved": gbs, "peak": peak, "unit": "GB/s",
-                     "frac": gbs / peak}
+                     "frac": gbs / peak, "peak_source": peak_src}
     if counters_apply and EXTEND_COUNTERS["l2_bytes_per_ray"]:
         l2b = EXTEND_COUNTERS["l2_bytes_per_ray"] * rays_per_launch
         l2_peak = l2_copy_gbs(torch)
@@ -813,9 +815,15 @@ def run_ours(args):
             "e2e": {"value": e2e, "unit": "Msamples/s", "h2d_bytes_per_step": 48,
                     "d2h_bytes_per_step": W_ * H_ * 12},
             "gpu_launches": launches,
-            "roofline": {"kernel": "k_extend (closest-hit traversal)", "bound": "hbm",
-                         "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_source": peak_src,
+            # the algorithmic bytes come through L1, whose data pipe is the unit
+            # the counters show fullest; DRAM and L2 have their own entries
+            "roofline": {"kernel": "k_extend_persistent (closest-hit traversal)",
+                         "bound": "latency",
+                         "bound_note": "dependent node loads at 32 warps an SM: issue slots (63-66 % "
+                                       "on the medium case), L1 (67-71 %), L2 and DRAM all have room",
+                         "achieved": achieved, "peak": L1_PEAK_GBS, "unit": "GB/s",
+                         "frac": achieved / L1_PEAK_GBS,
+                         "peak_source": "nominal: 148 SMs x 128 B of L1 data x 1.965 GHz",
                          "traffic": traffic,
                          "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum "
                                             "of k_extend_persistent per extend ray on the "
